@@ -212,13 +212,14 @@ __global__ void __launch_bounds__(128, CWPB_TRACE_MINB) k_trace_shade_rf(const _
     int err = 0;
     TravState<V, false, TRI> ray; typename TravState<V, false, TRI>::Stack stack;
     int k = -1; bool fin = false, drained = false;
+    const int cap = warp_share(n, gridDim.x * 4);
     for (;;) {
         if (__any_sync(0xffffffffu, fin)) {
             shade_path<PRIMARY>(a, P, fin, k, ray.o, ray.d, ray.hitT, ray.hitTri, ray.hu, ray.hv);
             if (fin) { k = -1; fin = false; }
         }
         if (!drained) {
-            const bool need = k < 0;
+            const bool need = k < 0 && lane < cap;
             const unsigned nm = __ballot_sync(0xffffffffu, need);
             if (nm) {
                 const int leader = __ffs(nm) - 1;
@@ -227,14 +228,99 @@ __global__ void __launch_bounds__(128, CWPB_TRACE_MINB) k_trace_shade_rf(const _
                 base = __shfl_sync(0xffffffffu, base, leader);
                 const int kk = base + __popc(nm & lanemask_lt());
                 if (need && kk < n) { k = kk; float3 o, d; float tmin; path_ray<PRIMARY>(a, P, k, o, d, tmin); ray.begin(o, d, tmin, 1e30f, 0); }
-                drained = __any_sync(0xffffffffu, need && kk >= n);   // the queue is empty from here on
+                drained = cap < 32 || __any_sync(0xffffffffu, need && kk >= n);   // the queue is empty from here on
             }
         }
-        if (!__any_sync(0xffffffffu, k >= 0)) break;
+        const unsigned held = __ballot_sync(0xffffffffu, k >= 0);
+        if (!held) break;
+        if constexpr (V == 8) {
+            if (drained && __popc(held) <= kGroupRays) { finish_groups(ray, held, k, fin, nodes, a.tv, stack, err); continue; }
+        }
         for (;;) {
             if (k >= 0 && !fin) fin = ray.step(nodes, a.tv, stack, err);
             const unsigned busy = __ballot_sync(0xffffffffu, k >= 0 && !fin);
-            if (!busy || (!drained && 32 - __popc(busy) >= CWPB_REFILL)) break;
+            if (!busy || (drained ? V == 8 && __popc(busy) <= kGroupRays : 32 - __popc(busy) >= CWPB_REFILL)) break;
+        }
+    }
+    if (err) atomicOr(a.err, err);
+}
+
+// Bounces over a CWBVH: persistent lanes with refill as above, with the warp's triangle tests shared out (test_leaves) and the
+// shading decoupled from the refill. Sharing pays while many lanes hold a ray, so the warp refills early; shading then would run
+// with a few lanes each time. Instead a finished ray leaves its path and triangle in a list in shared memory, and the warp
+// shades when the list is full, with all lanes: the ray is read from the queue again, and its distance and barycentrics come from one
+// more test of the triangle (the same arithmetic on the same operands, so the same bits). Camera rays keep k_trace_shade_rf: neighbouring
+// rays hit the same leaves in the same step, and sharing their tests measured 25% slower (34.8 vs 27.9 ms).
+#ifndef CWPB_BOUNCE_REFILL
+#define CWPB_BOUNCE_REFILL 6
+#endif
+struct BounceWarp { WarpLeaves<false> leaves; int2 done[32]; };   // done: (path, triangle or -1) of finished rays
+
+template <int TRI, bool STAGE = false>
+__global__ void __launch_bounds__(128, CWPB_TRACE_MINB) k_bounce(const __grid_constant__ KArgs a, const __grid_constant__ cwp_params P) {
+    __shared__ BounceWarp warps[4];
+    BounceWarp& w = warps[threadIdx.x >> 5];
+    const auto nodes = node_source<STAGE>(a);
+    int* const c = a.cnt + 4 * a.depth;
+    const int n = c[0];
+    const int lane = threadIdx.x & 31;
+    int err = 0, nDone = 0;
+    TravState<8, false, TRI> ray; typename TravState<8, false, TRI>::Stack stack;
+    int k = -1; bool fin = false, drained = false;
+    const int cap = warp_share(n, gridDim.x * 4);
+    for (;;) {
+        const unsigned fm = __ballot_sync(0xffffffffu, fin);
+        const bool last = drained && !__any_sync(0xffffffffu, k >= 0 && !fin);   // nothing left but the list
+        for (bool add = fm != 0; add || (last && nDone);) {
+            if (nDone + (add ? __popc(fm) : 33) > 32) {   // the list does not take them (or is the last): shade it
+                __syncwarp();
+                const bool valid = lane < nDone;
+                const int2 e = valid ? w.done[lane] : make_int2(0, -1);
+                float3 o = f3(0.f, 0.f, 0.f), d = f3(0.f, 0.f, 1.f); float tmin = 0.f, t = 1e30f, hu = 0.f, hv = 0.f; int tri = -1;
+                if (valid) {
+                    path_ray<false>(a, P, e.x, o, d, tmin);
+                    if (e.y >= 0) leaf_hit<false, TRI>(a.tv, e.y, 1, o, d, tmin, t, tri, hu, hv);
+                }
+                __syncwarp();
+                shade_path<false>(a, P, valid, e.x, o, d, t, tri, hu, hv);
+                nDone = 0;
+            }
+            if (!add) continue;
+            if (fin) { w.done[nDone + __popc(fm & lanemask_lt())] = make_int2(k, ray.hitTri); k = -1; fin = false; }
+            nDone += __popc(fm);
+            add = false;
+        }
+        if (!drained) {
+            const bool need = k < 0 && lane < cap;
+            const unsigned nm = __ballot_sync(0xffffffffu, need);
+            if (nm) {
+                const int leader = __ffs(nm) - 1;
+                int base = 0;
+                if (lane == leader) base = atomicAdd(c + 2, __popc(nm));
+                base = __shfl_sync(0xffffffffu, base, leader);
+                const int kk = base + __popc(nm & lanemask_lt());
+                if (need && kk < n) {
+                    k = kk; float3 o, d; float tmin; path_ray<false>(a, P, k, o, d, tmin); ray.begin(o, d, tmin, 1e30f, 0);
+                    w.leaves.ro[lane] = f4(o, tmin); w.leaves.rd[lane] = f4(d, 1e30f);
+                }
+                drained = cap < 32 || __any_sync(0xffffffffu, need && kk >= n);   // the queue is empty from here on
+            }
+        }
+        const unsigned held = __ballot_sync(0xffffffffu, k >= 0);
+        if (!held) { if (nDone == 0) break; drained = true; continue; }
+        if (drained && __popc(held) <= kGroupRays) {
+            ray.d = xyz(w.leaves.rd[lane]);   // (kept in shared memory alone until here)
+            finish_groups(ray, held, k, fin, nodes, a.tv, stack, err);
+            continue;
+        }
+        for (;;) {
+            const bool act = k >= 0 && !fin;
+            LeafSet set;
+            if (act) fin = ray.template visit<true>(nodes, a.tv, stack, set, err);
+            test_leaves<TRI, false>(w.leaves, set, a.tv, ray.hitT, ray.hitTri, ray.hu, ray.hv);
+            if (act && ray.node < 0) fin = true;
+            const unsigned busy = __ballot_sync(0xffffffffu, k >= 0 && !fin);
+            if (!busy || (drained ? __popc(busy) <= kGroupRays : 32 - __popc(busy) >= CWPB_BOUNCE_REFILL)) break;
         }
     }
     if (err) atomicOr(a.err, err);
@@ -277,6 +363,31 @@ __global__ void __launch_bounds__(128, CWPB_TRACE_MINB) k_shadow_rf(const __grid
     if (err) atomicOr(a.err, err);
 }
 
+static constexpr int kFewShadow = 8;   // rays per warp up to which shadow_few is taken (at 17 and more it measured 15-25% slower)
+// The shadow rays of a queue far too small to fill the GPU (CWBVH; ray k of this lane or -1): one ray per lane until at most
+// kGroupRays are left, then eight lanes per ray. A lit path's pixel and contribution are read when its ray is done. Not
+// inlined, so that the registers of the full queue's loop stay its own (inlined, it cost that loop 100 bytes of spills).
+template <int TRI, class N>
+__device__ __noinline__ void shadow_few(const KArgs& a, const N& nodes, int k, int& err) {
+    CwbvhTrav<true, TRI, -1> ray; typename CwbvhTrav<true, TRI, -1>::Stack stack;
+    bool fin = false;
+    if (k >= 0) ray.begin(xyz(__ldg(a.q.h0 + k)), xyz(__ldg(a.q.h1 + k)), 0.f, 1e30f, 0);
+    unsigned busy = __ballot_sync(0xffffffffu, k >= 0);
+    while (__popc(busy) > kGroupRays) {
+        if (k >= 0 && !fin) fin = ray.step(nodes, a.tv, stack, err);
+        busy = __ballot_sync(0xffffffffu, k >= 0 && !fin);
+    }
+    for (;;) {
+        if (fin && ray.hitTri < 0) {
+            const int pix = __float_as_int(__ldg(&a.q.h0[k].w)); const float2 h2 = __ldcs(a.q.h2 + k);
+            accum_add(a.accum, pix, f3(__ldg(&a.q.h1[k].w), h2.x, h2.y));
+        }
+        if (!busy) break;
+        finish_groups(ray, busy, k, fin, nodes, a.tv, stack, err);
+        busy = 0;
+    }
+}
+
 // FOCT >= 0 (CWBVH): the launch's shadow rays all point into octant FOCT (the sun's, when its cone stays inside one
 // octant), so their traversal takes the plane choice and child order as constants; a ray outside it (or with a zero
 // direction component) takes the per-ray form. Both visit the same nodes in the same order: the same result.
@@ -287,13 +398,16 @@ __global__ void __launch_bounds__(128, CWPB_TRACE_MINB) k_shadow(const __grid_co
     const int n = c[1];
     const int lane = threadIdx.x & 31;
     int err = 0;
+    int cap = warp_share(n, gridDim.x * 4);
+    if (V != 8 || cap > kFewShadow) cap = 32;
     for (;;) {
         int base = 0;
-        if (lane == 0) base = atomicAdd(c + 3, 32);
+        if (lane == 0) base = atomicAdd(c + 3, cap);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (base >= n) break;
-        const int k = base + lane;
-        if (k < n) {
+        const int k = lane < cap && base + lane < n ? base + lane : -1;
+        if constexpr (V == 8) { if (cap < 32) { shadow_few<TRI>(a, nodes, k, err); continue; } }
+        if (k >= 0) {
             const float4 h0 = __ldcs(a.q.h0 + k), h1 = __ldcs(a.q.h1 + k); const float2 h2 = __ldcs(a.q.h2 + k);
             float t = 1e30f, u, v; int tri = -1; bool hit;
             if constexpr (V == 8 && FOCT >= 0) {
@@ -408,13 +522,14 @@ template <class K> void prefer_l1(K*) {}
 
 template <int V, int TRI, bool STAGE = false> int occupancy_of(int& bt0, int& bt, int& bs, bool refill = false, size_t smem = 0) {
     if constexpr (!STAGE) {
-        if constexpr (V != 4) { prefer_l1(k_trace_shade_rf<V, TRI, true>); prefer_l1(k_trace_shade_rf<V, TRI, false>); prefer_l1(k_shadow_rf<V, TRI>); }
+        if constexpr (V != 4) { prefer_l1(k_trace_shade_rf<V, TRI, true>); if constexpr (V != 8) prefer_l1(k_trace_shade_rf<V, TRI, false>); prefer_l1(k_shadow_rf<V, TRI>); }
         prefer_l1(k_trace_shade<V, TRI, true>); prefer_l1(k_trace_shade<V, TRI, false>); prefer_l1(k_shadow<V, TRI>);
     }
     if constexpr (V != 4) {
         if (refill) {
             CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt0, k_trace_shade_rf<V, TRI, true, STAGE>, 128, smem));
-            CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, k_trace_shade_rf<V, TRI, false, STAGE>, 128, smem));
+            if constexpr (V == 8) CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, k_bounce<TRI, STAGE>, 128, smem));
+            else CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, k_trace_shade_rf<V, TRI, false, STAGE>, 128, smem));
             CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, k_shadow_rf<V, TRI, STAGE>, 128, smem));
             return CWP_OK;
         }
@@ -435,6 +550,7 @@ template <int V, int TRI, bool STAGE = false> void launch_depth(cwp_renderer* r,
     if constexpr (V != 4) {
         if (rf) {
             if (a.depth == 0) k_trace_shade_rf<V, TRI, true, STAGE><<<gt0, 128, sm, r->st>>>(a, r->P);
+            else if constexpr (V == 8) k_bounce<TRI, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
             else k_trace_shade_rf<V, TRI, false, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
         }
     }

@@ -167,15 +167,21 @@ __global__ void __launch_bounds__(kBatchBlock) k_trace_any(const float4* __restr
 #define CWPB_BATCH_REFILL 12
 #endif
 static constexpr int kRefillBatch = CWPB_BATCH_REFILL;
+static constexpr int kRefillShare = 6;   // with shared triangle tests (2 / 4 / 6 / 8 / 12 / 16 idle lanes: 1769 / 1690 / 1670 / 1683 / 1764 / 1896 us
+                                         // for 4.2 M incoherent closest hits)
 __device__ __forceinline__ unsigned lane_lt() { unsigned m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
 
 template <int V, int TRI, bool ANY>
 __global__ void __launch_bounds__(kBatchBlock, 8) k_trace_rf(const float4* __restrict__ nodes, const float4* __restrict__ tv, const float4* __restrict__ ro,
                                                              const float4* __restrict__ rd, float4* __restrict__ hits, int* __restrict__ occ, long long n, int* fetch, int* err) {
+    constexpr bool SHARE = V == 8 && !ANY;
+    __shared__ WarpLeaves<true> leaves[SHARE ? kBatchBlock / 32 : 1];
+    WarpLeaves<true>& ws = leaves[SHARE ? threadIdx.x >> 5 : 0];
     const int lane = threadIdx.x & 31;
     int e = 0;
     TravState<V, ANY, TRI> ray; typename TravState<V, ANY, TRI>::Stack stack;
     long long k = -1; bool fin = false, drained = false;
+    const int cap = warp_share(n, gridDim.x * (kBatchBlock / 32));
     for (;;) {
         if (fin) {
             if (ANY) __stcs(occ + k, ray.hitTri);
@@ -183,7 +189,7 @@ __global__ void __launch_bounds__(kBatchBlock, 8) k_trace_rf(const float4* __res
             k = -1; fin = false;
         }
         if (!drained) {
-            const bool need = k < 0;
+            const bool need = k < 0 && lane < cap;
             const unsigned nm = __ballot_sync(0xffffffffu, need);
             if (nm) {
                 const int leader = __ffs(nm) - 1;
@@ -191,15 +197,29 @@ __global__ void __launch_bounds__(kBatchBlock, 8) k_trace_rf(const float4* __res
                 if (lane == leader) base = atomicAdd((unsigned long long*)fetch, (unsigned long long)__popc(nm));
                 base = __shfl_sync(0xffffffffu, base, leader);
                 const long long kk = base + __popc(nm & lane_lt());
-                if (need && kk < n) { k = kk; const float4 O = __ldcs(ro + k), D = __ldcs(rd + k); ray.begin(xyz(O), xyz(D), O.w, D.w, 0); }
-                drained = __any_sync(0xffffffffu, need && kk >= n);
+                if (need && kk < n) { k = kk; const float4 O = __ldcs(ro + k), D = __ldcs(rd + k); ray.begin(xyz(O), xyz(D), O.w, D.w, 0); if constexpr (SHARE) { ws.ro[lane] = O; ws.rd[lane] = D; } }
+                drained = cap < 32 || __any_sync(0xffffffffu, need && kk >= n);
             }
         }
-        if (!__any_sync(0xffffffffu, k >= 0)) break;
+        const unsigned held = __ballot_sync(0xffffffffu, k >= 0);
+        if (!held) break;
+        if constexpr (V == 8) {
+            if (drained && __popc(held) <= kGroupRays) {
+                if constexpr (SHARE) ray.d = xyz(ws.rd[lane]);   // (kept in shared memory alone until here)
+                finish_groups(ray, held, k, fin, nodes, tv, stack, e);
+                continue;
+            }
+        }
         for (;;) {
-            if (k >= 0 && !fin) fin = ray.step(nodes, tv, stack, e);
+            if constexpr (SHARE) {
+                const bool act = k >= 0 && !fin;
+                LeafSet set;
+                if (act) fin = ray.template visit<true>(nodes, tv, stack, set, e);
+                test_leaves<TRI, true>(ws, set, tv, ray.hitT, ray.hitTri, ray.hu, ray.hv);
+                if (act && ray.node < 0) fin = true;
+            } else if (k >= 0 && !fin) fin = ray.step(nodes, tv, stack, e);
             const unsigned busy = __ballot_sync(0xffffffffu, k >= 0 && !fin);
-            if (!busy || (!drained && 32 - __popc(busy) >= kRefillBatch)) break;
+            if (!busy || (drained ? V == 8 && __popc(busy) <= kGroupRays : 32 - __popc(busy) >= (SHARE ? kRefillShare : kRefillBatch))) break;
         }
     }
     if (e) atomicOr(err, e);

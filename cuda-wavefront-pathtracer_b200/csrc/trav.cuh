@@ -16,6 +16,7 @@
 #pragma once
 #include "vecmath.h"
 #include <cuda_fp16.h>
+#include <type_traits>
 
 namespace cwpb {
 
@@ -225,6 +226,77 @@ __device__ __forceinline__ float qbyte(unsigned w, int s) {
     return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (unsigned)(s & 3))) - 8388608.0f;
 }
 
+// a * b + c of two floats at once (one instruction on sm_100), each rounded as fmaf
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+// ---- triangle tests shared over the warp (closest hits) ----
+// The rays' hit leaves of one node visit. Of a warp's 24 active rays about 9 hit a leaf per visit, of 1 to 3 triangles each:
+// tested by their own lanes, those run one dependent fetch and test after another with 3 lanes active, and took three
+// quarters of a visit's cycles (clock readings inside the kernel, 4.2 M incoherent rays over the 117k-triangle box field:
+// 1,580 cycles of node visit, 6,060 of leaf tests). test_leaves() lists the triangles of all lanes and hands them out 32 at a
+// time, one per lane, with the owner's ray read from shared memory: one fetch latency and one test for 16 triangles on
+// average. Measured there: 2,057 -> 1,670 us closest (12.1 -> 18.9 lanes per instruction, 449 -> 386 M instructions per
+// 1 M rays); rays and hits through shuffles instead of shared memory 1,781 us. Any-hit rays hit a quarter as many leaves
+// and stop at the first hit: for them the sharing measured no gain (434 vs 438 us) and their lanes test alone.
+struct LeafSet { unsigned hit = 0, m0 = 0, m1 = 0; int triBase = 0; };   // slots hit, the node's meta words, its first triangle
+template <bool UV>
+struct WarpLeaves {   // UV: hits with their barycentrics
+    typedef typename std::conditional<UV, float4, float2>::type Hit;
+    uint2 list[32];   // first triangle and owner of the leaf that starts at this position of the round
+    Hit res[32];      // (t, triangle) or (t, triangle, u, v) of the lanes whose test hit
+    float4 ro[32];    // each lane's ray: origin, tmin; direction, current hit distance
+    float4 rd[32];
+};
+__device__ __forceinline__ unsigned nibble_bytes(unsigned h) { return ((h * 0x00204081u) & 0x01010101u) * 255u; }   // bit i -> byte i full
+
+// All 32 lanes call it. Each ray gets the hit that testing its own triangles in slot order gives: the tests run against the
+// interval the ray had before the round, and the owner takes its hits in list order, a later one only when strictly closer.
+template <int TRI, bool UV>
+__device__ __forceinline__ void test_leaves(WarpLeaves<UV>& ws, const LeafSet& L, const float4* __restrict__ tv, float& hitT, int& hitTri, float& hu, float& hv) {
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    // triangles of this lane's leaves: the count fields (meta bits 5, 6) of the hit slots, summed by a multiply
+    const unsigned c0 = (((L.m0 >> 5) & 0x03030303u) + 0x01010101u) & nibble_bytes(L.hit & 15u), c1 = (((L.m1 >> 5) & 0x03030303u) + 0x01010101u) & nibble_bytes(L.hit >> 4);
+    const int cnt = (int)(((c0 + c1) * 0x01010101u) >> 24);
+    int incl = cnt;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) { const int v = __shfl_up_sync(all, incl, off); if (lane >= off) incl += v; }
+    const int total = __shfl_sync(all, incl, 31), p0 = incl - cnt;   // this lane's are [p0, incl) of the warp's list
+    for (int base = 0; base < total; base += 32) {
+        unsigned starts = 0;
+        int p = p0 - base;
+        for (unsigned h = L.hit; h; h &= h - 1) {
+            const int s = __ffs(h) - 1;
+            const unsigned m = byte_of(s < 4 ? L.m0 : L.m1, s);
+            const int c = (int)((m >> 5) & 3u) + 1;
+            if (p < 32 && p + c > 0) { const int q = max(p, 0); ws.list[q] = make_uint2((unsigned)(L.triBase + (int)(m & 31u) + q - p), (unsigned)lane); starts |= 1u << q; }
+            p += c;
+        }
+        starts = __reduce_or_sync(all, starts);
+        __syncwarp();
+        bool hit = false;
+        if (base + lane < total) {
+            const int at = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));   // the leaf this position belongs to
+            const uint2 e = ws.list[at];
+            const float4 O = ws.ro[e.y], D = ws.rd[e.y];
+            float t = D.w, u = 0.f, v = 0.f; int tri = -1;
+            leaf_hit<false, TRI>(tv, (int)e.x + lane - at, 1, xyz(O), xyz(D), O.w, t, tri, u, v);
+            hit = tri >= 0;
+            if (hit) { if constexpr (UV) ws.res[lane] = make_float4(t, __int_as_float(tri), u, v); else ws.res[lane] = make_float2(t, __int_as_float(tri)); }
+        }
+        const unsigned hits = __ballot_sync(all, hit);
+        if (hits) {
+            __syncwarp();
+            const int lo = max(p0 - base, 0), hi = min(incl - base, 32);
+            for (unsigned mine = hi > lo ? hits & ((0xffffffffu >> (32 - (hi - lo))) << lo) : 0u; mine; mine &= mine - 1) {
+                const auto r = ws.res[__ffs(mine) - 1];
+                if (r.x < hitT) { hitT = r.x; hitTri = __float_as_int(r.y); ws.rd[lane].w = r.x; if constexpr (UV) { hu = r.z; hv = r.w; } }
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // FOCT >= 0: every ray of the launch has direction octant FOCT and no zero direction component (the caller checks
 // per ray), so the near/far plane choice and the octant order are compile-time constants; -1: taken per ray
 template <bool ANY, int TRI, int FOCT>
@@ -240,6 +312,14 @@ struct CwbvhTrav {
     }
     template <class N, class S>
     __device__ __forceinline__ bool step(const N& nodes, const float4* __restrict__ tv, S& stack, int& err) {
+        LeafSet none;
+        return visit<false>(nodes, tv, stack, none, err);
+    }
+    // One node visit. SHARE = false: the hit leaves are tested here; true when the ray is finished. SHARE = true: they are
+    // returned in `leaves` for test_leaves(), the next node is chosen (node = -1 when none is left), and the ray is finished
+    // once its leaves are tested and node < 0; true when it stopped on a bound.
+    template <bool SHARE, class N, class S>
+    __device__ __forceinline__ bool visit(const N& nodes, const float4* __restrict__ tv, S& stack, LeafSet& leaves, int& err) {
         if (--budget < 0) { err |= kTravBudget; return true; }
         float4 nf[5]; fetch_node<5>(nodes, node, nf);
         const float4 f0 = nf[0], f1 = nf[1], f2 = nf[2], f3_ = nf[3], f4_ = nf[4];
@@ -267,21 +347,25 @@ struct CwbvhTrav {
         // factor 2^24 in their exponents (sx24 = 2^(e + 24) / d, exact), so fmaf(q 2^-24, sx24, ox) is bit for bit
         // fmaf(q, 2^e / d, ox) - the slab distances of the reference's decode - at one permute per two planes
         // instead of a permute and a subtraction per plane.
+        // SHARE: the two children of a permute go through one two-wide multiply-add (2% there; the any-hit kernels, which it
+        // costs spills, keep the scalar form)
         float2 pbx, pby, pbz, pcx, pcy, pcz;
 #pragma unroll
         for (int s = 0; s < 8; s++) {
-            float2 bx, by, bz, cx, cy, cz;
             if ((s & 1) == 0) {
                 const unsigned sel = (s & 2) ? 0x4342u : 0x4140u;
-                bx = __half22float2(h2_of_bits(__byte_perm(s < 4 ? nx0 : nx1, 0u, sel))); cx = __half22float2(h2_of_bits(__byte_perm(s < 4 ? px0 : px1, 0u, sel)));
-                by = __half22float2(h2_of_bits(__byte_perm(s < 4 ? ny0 : ny1, 0u, sel))); cy = __half22float2(h2_of_bits(__byte_perm(s < 4 ? py0 : py1, 0u, sel)));
-                bz = __half22float2(h2_of_bits(__byte_perm(s < 4 ? nz0 : nz1, 0u, sel))); cz = __half22float2(h2_of_bits(__byte_perm(s < 4 ? pz0 : pz1, 0u, sel)));
-                pbx = bx; pby = by; pbz = bz; pcx = cx; pcy = cy; pcz = cz;
+                pbx = __half22float2(h2_of_bits(__byte_perm(s < 4 ? nx0 : nx1, 0u, sel))); pcx = __half22float2(h2_of_bits(__byte_perm(s < 4 ? px0 : px1, 0u, sel)));
+                pby = __half22float2(h2_of_bits(__byte_perm(s < 4 ? ny0 : ny1, 0u, sel))); pcy = __half22float2(h2_of_bits(__byte_perm(s < 4 ? py0 : py1, 0u, sel)));
+                pbz = __half22float2(h2_of_bits(__byte_perm(s < 4 ? nz0 : nz1, 0u, sel))); pcz = __half22float2(h2_of_bits(__byte_perm(s < 4 ? pz0 : pz1, 0u, sel)));
+                if constexpr (SHARE) {
+                    const float2 sx = make_float2(sx24, sx24), sy = make_float2(sy24, sy24), sz = make_float2(sz24, sz24);
+                    const float2 o2x = make_float2(ox, ox), o2y = make_float2(oy, oy), o2z = make_float2(oz, oz);
+                    pbx = fma2(pbx, sx, o2x); pcx = fma2(pcx, sx, o2x); pby = fma2(pby, sy, o2y); pcy = fma2(pcy, sy, o2y); pbz = fma2(pbz, sz, o2z); pcz = fma2(pcz, sz, o2z);
+                }
             }
             const bool hi = s & 1;
-            const float xn = fmaf(hi ? pbx.y : pbx.x, sx24, ox), xf = fmaf(hi ? pcx.y : pcx.x, sx24, ox);
-            const float yn = fmaf(hi ? pby.y : pby.x, sy24, oy), yf = fmaf(hi ? pcy.y : pcy.x, sy24, oy);
-            const float zn = fmaf(hi ? pbz.y : pbz.x, sz24, oz), zf = fmaf(hi ? pcz.y : pcz.x, sz24, oz);
+            float xn = hi ? pbx.y : pbx.x, xf = hi ? pcx.y : pcx.x, yn = hi ? pby.y : pby.x, yf = hi ? pcy.y : pcy.x, zn = hi ? pbz.y : pbz.x, zf = hi ? pcz.y : pcz.x;
+            if constexpr (!SHARE) { xn = fmaf(xn, sx24, ox); xf = fmaf(xf, sx24, ox); yn = fmaf(yn, sy24, oy); yf = fmaf(yf, sy24, oy); zn = fmaf(zn, sz24, oz); zf = fmaf(zf, sz24, oz); }
             // entry = max(xn, yn, zn, tmin), exit = min(xf, yf, zf, hitT) selected with 3-input integer min/max on the
             // float bits: for values >= +0 the integer order is the float order, entry >= tmin >= +0, and any negative
             // candidate for the exit makes the float comparison below fail whichever negative value is picked - so
@@ -296,7 +380,8 @@ struct CwbvhTrav {
         if (oc & 1u) hits = ((hits & 0x55u) << 1) | ((hits & 0xAAu) >> 1);
         if (oc & 2u) hits = ((hits & 0x33u) << 2) | ((hits & 0xCCu) >> 2);
         if (oc & 4u) hits = ((hits & 0x0Fu) << 4) | ((hits & 0xF0u) >> 4);
-        while (leafHit) {
+        if constexpr (SHARE) { leaves.hit = leafHit; leaves.m0 = m0; leaves.m1 = m1; leaves.triBase = triBase; }
+        else while (leafHit) {
             const int s = __ffs(leafHit) - 1; leafHit &= leafHit - 1;
             const unsigned m = byte_of(s < 4 ? m0 : m1, s);
             if (leaf_hit<ANY, TRI>(tv, triBase + (int)(m & 31u), (int)((m >> 5) & 3u) + 1, o, d, tmin, hitT, hitTri, hu, hv) && ANY) return true;
@@ -305,14 +390,131 @@ struct CwbvhTrav {
             if (hm) { if (sp == kStack8) { err |= kTravOverflow; return true; } stack[sp++] = make_uint2(cb, (im << 8) | hm); }
             cb = (unsigned)childBase; im = imask; hm = hits;
         }
-        while (hm == 0) { if (sp == 0) return true; const uint2 e = stack[--sp]; cb = e.x; im = e.y >> 8; hm = e.y & 255u; }
+        while (hm == 0) { if (sp == 0) { node = -1; return !SHARE; } const uint2 e = stack[--sp]; cb = e.x; im = e.y >> 8; hm = e.y & 255u; }
         const unsigned k = __ffs(hm) - 1; hm &= hm - 1; const unsigned slot = k ^ oc;
         node = (int)cb + __popc(im & ((1u << slot) - 1u));
         return false;
     }
+
+    // ---- eight lanes per ray ----
+    // A ray alone in its warp (the stragglers of a drained queue, a batch of a few rays) is bound by the serial chain of its
+    // visits: node fetch, eight slab tests one after another, each hit triangle fetched and tested in turn. Here a group of
+    // eight lanes holds one ray, every field the same in all eight: lane j of the group tests the child of octant rank j
+    // (slot j ^ oct), so the group's ballot is the hit mask in visiting order, and tests that child's triangles when it is a
+    // leaf, all leaves of the node at once. The result is that of step(): the same nodes in the same order, and of a node's
+    // triangles the nearest hit (closest), ties to the lower slot, or the hit of the lowest slot (any).
+
+    // Takes over the at most four unfinished rays of the warp (lanes `busy`): group g the g-th of them, with its stack (every
+    // lane keeps a copy). Returns the lane the ray came from, or -1 for a group without one.
+    template <class S>
+    __device__ __forceinline__ int adopt8(unsigned busy, S& stack) {
+        const int lane = threadIdx.x & 31;
+        for (int g = lane >> 3; g > 0; g--) busy &= busy - 1;
+        const int from = __ffs(busy) - 1, src = from < 0 ? lane : from;
+        const unsigned all = 0xffffffffu;
+        o.x = __shfl_sync(all, o.x, src); o.y = __shfl_sync(all, o.y, src); o.z = __shfl_sync(all, o.z, src);
+        d.x = __shfl_sync(all, d.x, src); d.y = __shfl_sync(all, d.y, src); d.z = __shfl_sync(all, d.z, src);
+        idx = safe_rcp(d.x); idy = safe_rcp(d.y); idz = safe_rcp(d.z);
+        tmin = __shfl_sync(all, tmin, src); hitT = __shfl_sync(all, hitT, src); hu = __shfl_sync(all, hu, src); hv = __shfl_sync(all, hv, src);
+        hitTri = __shfl_sync(all, hitTri, src); node = __shfl_sync(all, node, src); budget = __shfl_sync(all, budget, src);
+        oct = (d.x > 0.f ? 1u : 0u) | (d.y > 0.f ? 2u : 0u) | (d.z > 0.f ? 4u : 0u);
+        cb = __shfl_sync(all, cb, src); im = __shfl_sync(all, im, src); hm = __shfl_sync(all, hm, src);
+        sp = __shfl_sync(all, sp, src);
+        if (from < 0) sp = 0;   // (a lane that never held a ray)
+        const int top = (int)__reduce_max_sync(all, (unsigned)sp);
+        for (int i = 0; i < top; i++) {   // entry i of every lane is read before it is overwritten
+            uint2 e = stack[i];
+            e.x = __shfl_sync(all, e.x, src); e.y = __shfl_sync(all, e.y, src);
+            stack[i] = e;
+        }
+        return from;
+    }
+    // One node visit of every group with act set (the same in its eight lanes); all 32 lanes call it. True when the group's
+    // ray is finished.
+    template <class S>
+    __device__ __forceinline__ bool step8(bool act, const float4* __restrict__ nodes, const float4* __restrict__ tv, S& stack, int& err) {
+        const unsigned all = 0xffffffffu;
+        const int lane = threadIdx.x & 31, gs = lane & 24;
+        const unsigned slot = (unsigned)(lane & 7) ^ oct;
+        bool fin = false;
+        if (act && --budget < 0) { err |= kTravBudget; act = false; fin = true; }
+        bool inner = false, leaf = false;
+        int childBase = 0, triBase = 0; unsigned imask = 0, meta = 0;
+        if (act) {
+            const float4* nb = nodes + 5 * (size_t)node;
+            const unsigned char* q = reinterpret_cast<const unsigned char*>(nb + 2) + slot;   // lo x, lo y, lo z, hi x, hi y, hi z: 8 bytes each
+            const int ax = idx < 0.f ? 24 : 0, ay = idy < 0.f ? 24 : 0, az = idz < 0.f ? 24 : 0;
+            const float4 f0 = ld4(nb), f1 = ld4(nb + 1);
+            const unsigned qxn = __ldg(q + ax), qxf = __ldg(q + 24 - ax), qyn = __ldg(q + 8 + ay), qyf = __ldg(q + 32 - ay), qzn = __ldg(q + 16 + az), qzf = __ldg(q + 40 - az);
+            const unsigned ew = __float_as_uint(f0.w);
+            const float sx = __uint_as_float((ew & 255u) << 23) * idx, sy = __uint_as_float(((ew >> 8) & 255u) << 23) * idy, sz = __uint_as_float(((ew >> 16) & 255u) << 23) * idz;
+            const float ox = (f0.x - o.x) * idx, oy = (f0.y - o.y) * idy, oz = (f0.z - o.z) * idz;
+            imask = ew >> 24; childBase = __float_as_int(f1.x); triBase = __float_as_int(f1.y);
+            meta = byte_of(__float_as_uint(slot < 4 ? f1.z : f1.w), (int)slot);
+            const float xn = fmaf((float)qxn, sx, ox), yn = fmaf((float)qyn, sy, oy), zn = fmaf((float)qzn, sz, oz);
+            const float xf = fmaf((float)qxf, sx, ox), yf = fmaf((float)qyf, sy, oy), zf = fmaf((float)qzf, sz, oz);
+            const float tn = __int_as_float(__vimax3_s32(__float_as_int(xn), __float_as_int(yn), max(__float_as_int(zn), __float_as_int(tmin))));
+            const float tf = __int_as_float(__vimin3_s32(__float_as_int(xf), __float_as_int(yf), min(__float_as_int(zf), __float_as_int(hitT))));
+            const bool hit = tn <= tf;
+            inner = hit && ((imask >> slot) & 1u); leaf = hit && (meta & 0x80u);
+        }
+        const unsigned innerB = __ballot_sync(all, inner);
+        if (__ballot_sync(all, leaf)) {
+            float bt = hitT, bu = 0.f, bv = 0.f; int bi = -1;
+            if (leaf) leaf_hit<ANY, TRI>(tv, triBase + (int)(meta & 31u), (int)((meta >> 5) & 3u) + 1, o, d, tmin, bt, bi, bu, bv);
+            if (__ballot_sync(all, bi >= 0)) {
+                float kt = ANY ? 0.f : (bi >= 0 ? bt : INFINITY); unsigned ks = bi >= 0 ? slot : 8u;
+#pragma unroll
+                for (int off = 1; off < 8; off <<= 1) {
+                    const float ot = ANY ? 0.f : __shfl_xor_sync(all, kt, off); const unsigned os = __shfl_xor_sync(all, ks, off);
+                    if (ot < kt || (ot == kt && os < ks)) { kt = ot; ks = os; }
+                }
+                const int src = ks < 8u ? gs | (int)(ks ^ oct) : lane;
+                const float wt = __shfl_sync(all, bt, src), wu = __shfl_sync(all, bu, src), wv = __shfl_sync(all, bv, src); const int wi = __shfl_sync(all, bi, src);
+                if (ks < 8u) { hitT = wt; hu = wu; hv = wv; hitTri = wi; if (ANY) { act = false; fin = true; } }
+            }
+        }
+        if (act) {
+            const unsigned hits = (innerB >> gs) & 255u;
+            if (hits) {
+                if (hm) { if (sp == kStack8) { err |= kTravOverflow; return true; } stack[sp++] = make_uint2(cb, (im << 8) | hm); }
+                cb = (unsigned)childBase; im = imask; hm = hits;
+            }
+            while (hm == 0) { if (sp == 0) return true; const uint2 e = stack[--sp]; cb = e.x; im = e.y >> 8; hm = e.y & 255u; }
+            const unsigned k = __ffs(hm) - 1; hm &= hm - 1; const unsigned s = k ^ oct;
+            node = (int)cb + __popc(im & ((1u << s) - 1u));
+        }
+        return fin;
+    }
 };
 
 template <bool ANY, int TRI> struct TravState<8, ANY, TRI> : CwbvhTrav<ANY, TRI, -1> {};
+
+__device__ __forceinline__ const float4* global_nodes(const float4* n) { return n; }
+__device__ __forceinline__ const float4* global_nodes(const StagedNodes& n) { return n.g; }
+
+// Items of an n-item queue that one of `warps` resident warps takes at a time: 32, or, when the queue does not fill them all,
+// an equal share in one fetch (a warp with fewer rays runs each of them faster: less divergence, and groups from the start)
+__device__ __forceinline__ int warp_share(long long n, unsigned warps) {
+    return n >= 32ll * warps ? 32 : (int)((unsigned)n + warps - 1) / (int)warps;
+}
+
+static constexpr int kGroupRays = 4;   // unfinished rays a warp can hold with eight lanes each
+
+// Runs the at most kGroupRays unfinished rays of a warp (lanes `busy`, each holding item k) to their end, eight lanes per ray.
+// On return the first lane of each group that had one holds the ray, its item k and fin = true; the other lanes hold none.
+template <class T, class N, class S, class K>
+__device__ __forceinline__ void finish_groups(T& ray, unsigned busy, K& k, bool& fin, const N& nodes, const float4* __restrict__ tv, S& stack, int& err) {
+    const int lane = threadIdx.x & 31;
+    const int from = ray.adopt8(busy, stack);
+    const K item = __shfl_sync(0xffffffffu, k, from < 0 ? lane : from);
+    bool act = from >= 0;
+    const bool had = act;
+    const float4* const g = global_nodes(nodes);
+    while (__any_sync(0xffffffffu, act)) { if (ray.step8(act, g, tv, stack, err)) act = false; }
+    fin = had && (lane & 7) == 0;
+    k = fin ? item : (K)-1;
+}
 
 // direction octant of d (bit i set: component i positive), or -1 when a component is zero (its sign then decides the
 // plane choice, not the octant bit)
