@@ -36,6 +36,7 @@ struct KArgs {
     const float4* nodes; const float4* tv; const float4* tris; const float4* nrm; const float3* albedo;
     Queues q; float4* accum; int* cnt; int* err;
     int nk, N, sBase, depth;
+    const int* sDev;   // null, or a device word added to sBase: the first sample of the frame, so that one captured graph serves every range
     int staged;   // CWBVH nodes each block copies into shared memory (the first `staged`, i.e. the top levels)
 };
 
@@ -52,6 +53,7 @@ __device__ __forceinline__ auto node_source(const KArgs& a) {
     } else return a.nodes;
 }
 
+__device__ __forceinline__ int sample_base(const KArgs& a) { return a.sBase + (a.sDev ? __ldg(a.sDev) : 0); }
 __device__ __forceinline__ float rnd(const cwp_params& P, unsigned pix, unsigned smp, unsigned depth, unsigned dim) { return sample01(pix, smp, depth, dim, P.seed); }
 __device__ __forceinline__ float3 v3(const float* a) { return f3(a[0], a[1], a[2]); }
 __device__ __forceinline__ unsigned lanemask_lt() { unsigned m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
@@ -121,7 +123,7 @@ __device__ __forceinline__ void shade_path(const KArgs& a, const cwp_params& P, 
             id = __float_as_int(__ldg(&a.q.s0[rd][k].w)); const float tr = __ldg(&a.q.s1[rd][k].w); const float2 s2 = __ldcs(a.q.s2[rd] + k);
             T = f3(tr, s2.x, s2.y);
         }
-        pix = tile_pixel(id % a.N, P.cam.w, P.cam.h); smp = (unsigned)(a.sBase + id / a.N);
+        pix = tile_pixel(id % a.N, P.cam.w, P.cam.h); smp = (unsigned)(sample_base(a) + id / a.N);
     }
     bool wantShadow = false, wantCont = false;
     float3 po = o, l = d, contrib = T, nd = d;
@@ -166,7 +168,7 @@ __device__ __forceinline__ void shade_path(const KArgs& a, const cwp_params& P, 
 // the ray of path k at this depth: camera ray (depth 0) or the queued continuation
 template <bool PRIMARY>
 __device__ __forceinline__ void path_ray(const KArgs& a, const cwp_params& P, int k, float3& o, float3& d, float& tmin) {
-    if (PRIMARY) { int pix; unsigned smp; camera_ray(P, k, a.N, a.sBase, o, d, pix, smp); tmin = P.near_clip; }
+    if (PRIMARY) { int pix; unsigned smp; camera_ray(P, k, a.N, sample_base(a), o, d, pix, smp); tmin = P.near_clip; }
     else { const int rd = a.depth & 1; const float4 s0 = __ldcs(a.q.s0[rd] + k), s1 = __ldcs(a.q.s1[rd] + k); o = xyz(s0); d = xyz(s1); tmin = 0.f; }
 }
 
@@ -503,9 +505,12 @@ struct cwp_renderer {
     std::vector<unsigned long long> htot;                 // last frame's per-depth totals
     std::vector<cudaEvent_t> ev; int evPasses = 0;        // profiling: 4 events per (pass, depth)
     std::vector<float> traceMs, shadowMs;                 // last frame's per-depth kernel times
-    int* hcnt = nullptr;   // pinned copy of the counters (host loop)
+    int* hcnt = nullptr;   // pinned: copy of the counters (host loop), then the first sample, then the frame's totals and status
     cudaStream_t st = nullptr; cudaEvent_t f0 = nullptr, f1 = nullptr;
-    cudaGraphExec_t gexec = nullptr; int gSpp = -1, gBase = 0;
+    // Shadow passes beside the next bounce: in a captured frame whose passes are small enough for a shadow queue per depth, the
+    // shadow rays of a depth run on a second stream while the next depth is traced (see enqueue_passes)
+    bool beside = false; cudaStream_t st2 = nullptr; cudaEvent_t traced = nullptr, shadowed = nullptr;
+    cudaGraphExec_t gexec = nullptr; int gSpp = -1;
     int gridTrace = 0, gridTrace0 = 0, gridShadow = 0, nSM = 0; bool refill = false, refillShadow = false;
     int staged = 0;   // CWBVH nodes staged in each traversal block's shared memory (0 = none)
     std::vector<void*> allocs;
@@ -541,7 +546,9 @@ template <int V, int TRI, bool STAGE = false> int occupancy_of(int& bt0, int& bt
 }
 
 // ev: 4 events (trace start/end, shadow start/end) or nullptr
-template <int V, int TRI, bool STAGE = false> void launch_depth(cwp_renderer* r, KArgs a, int gt0, int gt, int gs, cudaEvent_t* ev) {
+template <int V, int TRI, bool STAGE = false> void launch_depth(cwp_renderer* r, KArgs a, int gt0, int gt, int gs, cudaEvent_t* ev, bool beside) {
+    const cudaStream_t ss = beside ? r->st2 : r->st;   // the shadow pass's stream
+    const bool shadows = a.depth + 1 < r->depths;      // a path's last hit (depth bounces + 1) casts none
     // external records: inside a stream capture they become event-record nodes of the graph
     bool rf = false, rfShadow = false;
     const size_t sm = STAGE ? (size_t)80 * a.staged : 0;
@@ -567,15 +574,16 @@ template <int V, int TRI, bool STAGE = false> void launch_depth(cwp_renderer* r,
         k_sort_scatter<<<r->nSM * 8, 256, 0, r->st>>>(sa);
     }
     if (ev) { cudaEventRecordWithFlags(ev[1], r->st, cudaEventRecordExternal); cudaEventRecordWithFlags(ev[2], r->st, cudaEventRecordExternal); }
-    if constexpr (V != 4) { if (rfShadow) k_shadow_rf<V, TRI, STAGE><<<gs, 128, sm, r->st>>>(a); }
-    if (!rfShadow) {
+    if (beside) { cudaEventRecord(r->traced, r->st); cudaStreamWaitEvent(r->st2, r->traced, 0); }
+    if constexpr (V != 4) { if (rfShadow && shadows) k_shadow_rf<V, TRI, STAGE><<<gs, 128, sm, ss>>>(a); }
+    if (!rfShadow && shadows) {
         int foct = -1;
         if constexpr (V == 8 && !STAGE) foct = sun_octant(r->P);
         switch (foct) {
-#define CWPB_SO(F) case F: if constexpr (V == 8 && !STAGE) k_shadow<8, TRI, false, F><<<gs, 128, sm, r->st>>>(a); break;
+#define CWPB_SO(F) case F: if constexpr (V == 8 && !STAGE) k_shadow<8, TRI, false, F><<<gs, 128, sm, ss>>>(a); break;
             CWPB_SO(0) CWPB_SO(1) CWPB_SO(2) CWPB_SO(3) CWPB_SO(4) CWPB_SO(5) CWPB_SO(6) CWPB_SO(7)
 #undef CWPB_SO
-            default: k_shadow<V, TRI, STAGE><<<gs, 128, sm, r->st>>>(a);
+            default: k_shadow<V, TRI, STAGE><<<gs, 128, sm, ss>>>(a);
         }
     }
     if (ev) cudaEventRecordWithFlags(ev[3], r->st, cudaEventRecordExternal);
@@ -588,14 +596,15 @@ KArgs base_args(cwp_renderer* r) {
     return a;
 }
 
-void dispatch_depth(cwp_renderer* r, KArgs a, int gt0, int gt, int gs, int pass) {
+void dispatch_depth(cwp_renderer* r, KArgs a, int gt0, int gt, int gs, int pass, bool beside = false) {
+    if (beside) { const size_t at = (size_t)a.depth * r->nk; a.q.h0 += at; a.q.h1 += at; a.q.h2 += at; }   // the depth's own shadow queue
     const int V = r->scene.variant, T = r->scene.tri;
     if (r->O.sort && a.depth > 0) { const int rd = a.depth & 1; a.q.s0[rd] = r->t0; a.q.s1[rd] = r->t1; a.q.s2[rd] = r->t2; }
     cudaEvent_t* ev = r->O.profile ? &r->ev[((size_t)pass * r->depths + a.depth) * 4] : nullptr;
-    if (V == 2) { if (T) launch_depth<2, 1>(r, a, gt0, gt, gs, ev); else launch_depth<2, 0>(r, a, gt0, gt, gs, ev); }
-    else if (V == 4) { if (T) launch_depth<4, 1>(r, a, gt0, gt, gs, ev); else launch_depth<4, 0>(r, a, gt0, gt, gs, ev); }
-    else if (r->staged) { if (T) launch_depth<8, 1, true>(r, a, gt0, gt, gs, ev); else launch_depth<8, 0, true>(r, a, gt0, gt, gs, ev); }
-    else { if (T) launch_depth<8, 1>(r, a, gt0, gt, gs, ev); else launch_depth<8, 0>(r, a, gt0, gt, gs, ev); }
+    if (V == 2) { if (T) launch_depth<2, 1>(r, a, gt0, gt, gs, ev, beside); else launch_depth<2, 0>(r, a, gt0, gt, gs, ev, beside); }
+    else if (V == 4) { if (T) launch_depth<4, 1>(r, a, gt0, gt, gs, ev, beside); else launch_depth<4, 0>(r, a, gt0, gt, gs, ev, beside); }
+    else if (r->staged) { if (T) launch_depth<8, 1, true>(r, a, gt0, gt, gs, ev, beside); else launch_depth<8, 0, true>(r, a, gt0, gt, gs, ev, beside); }
+    else { if (T) launch_depth<8, 1>(r, a, gt0, gt, gs, ev, beside); else launch_depth<8, 0>(r, a, gt0, gt, gs, ev, beside); }
 }
 
 // profiling events for `passes` passes (created on first need, kept)
@@ -606,13 +615,23 @@ int ensure_events(cwp_renderer* r, int passes) {
     return CWP_OK;
 }
 
-// all passes of a frame with device-side queue lengths and persistent grids (the captured sequence)
-int enqueue_passes(cwp_renderer* r, int spp, int sBase) {
+// All passes of a frame with device-side queue lengths and persistent grids (the captured sequence). Every launch of a small
+// pass ends in a tail: its queue is empty and a few long rays hold the GPU. With r->beside the shadow pass of a depth is a
+// branch of the graph beside the next depth's trace+shade, on a stream of lower priority, and fills that tail; the branches
+// join at the end of the pass. It needs a shadow queue per depth, so it is taken up to kBesideEntries queue entries (672 MB);
+// larger passes lose under 1% to tails.
+static constexpr long long kBesideEntries = 1ll << 24;
+int enqueue_passes(cwp_renderer* r, int spp) {
     const int nInts = 4 * (r->depths + 1);
-    for (int s = sBase, pass = 0; s < sBase + spp; s += r->K, pass++) {
+    const bool beside = r->beside && !r->O.profile;   // (per-kernel times need the kernels one after another)
+    for (int s = 0, pass = 0; s < spp; s += r->K, pass++) {
         k_pass_begin<<<1, 128, 0, r->st>>>(r->cnt, nInts, (int)r->nk, r->sortBins, r->sortBins ? 2 * kSortBins * r->depths : 0);
-        KArgs a = base_args(r); a.sBase = s;
-        for (int d = 0; d < r->depths; d++) { a.depth = d; dispatch_depth(r, a, r->gridTrace0, r->gridTrace, r->gridShadow, pass); }
+        KArgs a = base_args(r); a.sBase = s; a.sDev = r->cnt + nInts;
+        for (int d = 0; d < r->depths; d++) {
+            a.depth = d;
+            dispatch_depth(r, a, r->gridTrace0, r->gridTrace, r->gridShadow, pass, beside && d < r->depths - 1);
+        }
+        if (beside) { CWPB_CUDA(cudaEventRecord(r->shadowed, r->st2)); CWPB_CUDA(cudaStreamWaitEvent(r->st, r->shadowed, 0)); }
         k_pass_end<<<1, 32, 0, r->st>>>(r->cnt, r->depths, r->tot);
     }
     CWPB_CUDA(cudaGetLastError());
@@ -649,6 +668,9 @@ extern "C" void cwp_renderer_destroy(cwp_renderer* r) {
     if (r->st) cudaStreamDestroy(r->st);
     if (r->f0) cudaEventDestroy(r->f0);
     if (r->f1) cudaEventDestroy(r->f1);
+    if (r->st2) cudaStreamDestroy(r->st2);
+    if (r->traced) cudaEventDestroy(r->traced);
+    if (r->shadowed) cudaEventDestroy(r->shadowed);
     delete r;
 }
 
@@ -668,7 +690,16 @@ extern "C" int cwp_renderer_init(cwp_renderer* r, const cwp_params* p, const cwp
     CWPB_CHECK(r->scene.variant == o->variant, CWP_ERR_INVALID, "options.variant %d does not match the node stride (layout %d)", o->variant, r->scene.variant);
     r->P = *p; r->O = *o;
     r->N = p->cam.w * p->cam.h; r->K = o->batch; r->nk = nk; r->depths = o->bounces + 2;
-    if (!r->st) { CWPB_CUDA(cudaStreamCreateWithFlags(&r->st, cudaStreamNonBlocking)); CWPB_CUDA(cudaEventCreate(&r->f0)); CWPB_CUDA(cudaEventCreate(&r->f1)); }
+    if (!r->shadowed) {
+        int least = 0, greatest = 0;
+        CWPB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        if (!r->st) CWPB_CUDA(cudaStreamCreateWithPriority(&r->st, cudaStreamNonBlocking, greatest < least ? least - 1 : least));
+        if (!r->f0) CWPB_CUDA(cudaEventCreate(&r->f0));
+        if (!r->f1) CWPB_CUDA(cudaEventCreate(&r->f1));
+        if (!r->st2) CWPB_CUDA(cudaStreamCreateWithPriority(&r->st2, cudaStreamNonBlocking, least));
+        if (!r->traced) CWPB_CUDA(cudaEventCreateWithFlags(&r->traced, cudaEventDisableTiming));
+        CWPB_CUDA(cudaEventCreateWithFlags(&r->shadowed, cudaEventDisableTiming));
+    }
     auto alloc = [&](void** dst, size_t bytes) -> int {
         cudaError_t e = cudaMalloc(dst, bytes);
         if (e != cudaSuccess) { release(r); return set_error(CWP_ERR_NOMEM, "cannot allocate %.1f MB of path state: %s", bytes / 1e6, cudaGetErrorString(e)); }
@@ -693,16 +724,28 @@ extern "C" int cwp_renderer_init(cwp_renderer* r, const cwp_params* p, const cwp
         r->boxLo = f3(lo[0], lo[1], lo[2]);
         r->boxInv = f3(4.f / std::max(hi[0] - lo[0], 1e-30f), 4.f / std::max(hi[1] - lo[1], 1e-30f), 4.f / std::max(hi[2] - lo[2], 1e-30f));
     }
-    if (!rc) rc = alloc((void**)&r->q.h0, NK * 16);
-    if (!rc) rc = alloc((void**)&r->q.h1, NK * 16);
-    if (!rc) rc = alloc((void**)&r->q.h2, NK * 8);
     if (!rc) rc = alloc((void**)&r->accum, (size_t)r->N * 16);
-    if (!rc) rc = alloc((void**)&r->cnt, (size_t)4 * (r->depths + 1) * sizeof(int));
-    if (!rc) rc = alloc((void**)&r->err, sizeof(int));
-    if (!rc) rc = alloc((void**)&r->tot, 2 * (size_t)r->depths * sizeof(unsigned long long));
+    if (!rc) rc = alloc((void**)&r->cnt, ((size_t)4 * (r->depths + 1) + 1) * sizeof(int));   // and the frame's first sample
+    if (!rc) rc = alloc((void**)&r->tot, (2 * (size_t)r->depths + 1) * sizeof(unsigned long long));   // and the status word
     if (rc) return rc;
-    CWPB_CUDA(cudaMallocHost(&r->hcnt, (size_t)4 * (r->depths + 1) * sizeof(int)));
-    CWPB_CUDA(cudaMemset(r->err, 0, sizeof(int)));
+    r->err = reinterpret_cast<int*>(r->tot + 2 * r->depths);
+    // shadow queues: one per depth where shadow passes run beside the next bounce and the memory is there, else one
+    r->beside = false;
+    if (o->graph && o->bounces >= 1 && nk * (o->bounces + 1) <= kBesideEntries) {
+        const size_t NE = NK * (o->bounces + 1); void* h = nullptr;
+        if (cudaMalloc(&h, NE * 40) == cudaSuccess) {
+            r->allocs.push_back(h); r->beside = true;
+            r->q.h0 = (float4*)h; r->q.h1 = r->q.h0 + NE; r->q.h2 = (float2*)(r->q.h1 + NE);
+        } else cudaGetLastError();
+    }
+    if (!r->beside) {
+        rc = alloc((void**)&r->q.h0, NK * 16);
+        if (!rc) rc = alloc((void**)&r->q.h1, NK * 16);
+        if (!rc) rc = alloc((void**)&r->q.h2, NK * 8);
+        if (rc) return rc;
+    }
+    CWPB_CUDA(cudaMallocHost(&r->hcnt, ((size_t)4 * (r->depths + 1) + 2) * sizeof(int) + (2 * (size_t)r->depths + 1) * sizeof(unsigned long long)));
+    CWPB_CUDA(cudaMemset(r->tot, 0, (2 * (size_t)r->depths + 1) * sizeof(unsigned long long)));
     CWPB_CUDA(cudaMemset(r->accum, 0, (size_t)r->N * 16));
     size_t free1 = 0; CWPB_CUDA(cudaMemGetInfo(&free1, &total));
     r->vramMB = (double)(free0 - free1) / 1048576.0;
@@ -757,25 +800,29 @@ extern "C" int cwp_renderer_render(cwp_renderer* r, int32_t spp, cwp_frame_stats
         if (r->gexec) { CWPB_CUDA(cudaGraphExecDestroy(r->gexec)); r->gexec = nullptr; r->gSpp = -1; }   // events are captured nodes
         if (int rc = ensure_events(r, passes)) return rc;
     }
+    const int nInts = 4 * (r->depths + 1);
+    if (r->O.graph) {   // the frame's first sample is data, so frames of the same sample count share the captured graph
+        r->hcnt[nInts] = sBase;
+        CWPB_CUDA(cudaMemcpyAsync(r->cnt + nInts, r->hcnt + nInts, sizeof(int), cudaMemcpyHostToDevice, r->st));
+    }
     CWPB_CUDA(cudaEventRecord(r->f0, r->st));
     if (r->O.graph) {
-        if (!r->gexec || r->gSpp != spp || r->gBase != sBase) {   // the sample range is part of the captured launches
+        if (!r->gexec || r->gSpp != spp) {
             if (r->gexec) { CWPB_CUDA(cudaGraphExecDestroy(r->gexec)); r->gexec = nullptr; }
             cudaGraph_t g;
             CWPB_CUDA(cudaStreamBeginCapture(r->st, cudaStreamCaptureModeThreadLocal));
-            int rc = enqueue_passes(r, spp, sBase);
+            int rc = enqueue_passes(r, spp);
             cudaError_t e = cudaStreamEndCapture(r->st, &g);
             if (rc) { if (e == cudaSuccess) cudaGraphDestroy(g); return rc; }
             CWPB_CUDA(e);
             e = cudaGraphInstantiate(&r->gexec, g, 0);
             cudaGraphDestroy(g);
             CWPB_CUDA(e);
-            r->gSpp = spp; r->gBase = sBase;
+            r->gSpp = spp;
         }
         CWPB_CUDA(cudaGraphLaunch(r->gexec, r->st));
     } else {
         // host loop: exact grids from the queue lengths read back after each depth (one sync per bounce)
-        const int nInts = 4 * (r->depths + 1);
         for (int s = sBase, pass = 0; s < sBase + spp; s += r->K, pass++) {
             k_pass_begin<<<1, 128, 0, r->st>>>(r->cnt, nInts, (int)r->nk, r->sortBins, r->sortBins ? 2 * kSortBins * r->depths : 0);
             KArgs a = base_args(r); a.sBase = s;
@@ -795,12 +842,13 @@ extern "C" int cwp_renderer_render(cwp_renderer* r, int32_t spp, cwp_frame_stats
         CWPB_CUDA(cudaGetLastError());
     }
     CWPB_CUDA(cudaEventRecord(r->f1, r->st));
-    CWPB_CUDA(cudaEventSynchronize(r->f1));
+    // totals and status in one copy behind the frame, one wait for both
+    unsigned long long* const ht = reinterpret_cast<unsigned long long*>(r->hcnt + nInts + 2);   // (nInts + 2 is even: 8-byte aligned)
+    CWPB_CUDA(cudaMemcpyAsync(ht, r->tot, (2 * (size_t)r->depths + 1) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, r->st));
+    CWPB_CUDA(cudaStreamSynchronize(r->st));
     float ms = 0.f; CWPB_CUDA(cudaEventElapsedTime(&ms, r->f0, r->f1));
-    int herr = 0;
-    r->htot.assign(2 * (size_t)r->depths, 0);
-    CWPB_CUDA(cudaMemcpy(r->htot.data(), r->tot, r->htot.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
-    CWPB_CUDA(cudaMemcpy(&herr, r->err, sizeof(int), cudaMemcpyDeviceToHost));
+    r->htot.assign(ht, ht + 2 * (size_t)r->depths);
+    const int herr = (int)(unsigned)ht[2 * (size_t)r->depths];
     double rays = 0, shadow = 0;
     for (int d = 0; d < r->depths; d++) { rays += (double)r->htot[2 * d]; shadow += (double)r->htot[2 * d + 1]; }
     st->frame_ms = ms; st->trace_ms = ms; st->rays = rays; st->shadow_rays = shadow;
@@ -979,7 +1027,7 @@ extern "C" int cwp_render_noalloc(const cwp_params* p, const cwp_device_scene* s
             a.depth = d;
 #define CWPB_NA(VV, TT) do { if (d == 0) k_trace_shade<VV, TT, true><<<na.gridTrace0, 128, 0, st>>>(a, *p); \
                              else k_trace_shade<VV, TT, false><<<na.gridTrace, 128, 0, st>>>(a, *p); \
-                             k_shadow<VV, TT><<<na.gridShadow, 128, 0, st>>>(a); } while (0)
+                             if (d + 1 < depths) k_shadow<VV, TT><<<na.gridShadow, 128, 0, st>>>(a); } while (0)
             if (o->variant == 2) { if (o->tri) CWPB_NA(2, 1); else CWPB_NA(2, 0); }
             else if (o->variant == 4) { if (o->tri) CWPB_NA(4, 1); else CWPB_NA(4, 0); }
             else { if (o->tri) CWPB_NA(8, 1); else CWPB_NA(8, 0); }
