@@ -589,7 +589,10 @@ template <int V, int TRI, bool STAGE = false> int occupancy_of(int& bt0, int& bt
     }
     if constexpr (V != 4) {
         if (refill) {
+            int b0 = 0;   // camera rays: one fetch per warp, or refill when it is asked for; one grid fits both
             CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt0, k_trace_shade_rf<V, TRI, true, STAGE>, 128, smem));
+            CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_trace_shade<V, TRI, true, STAGE>, 128, smem));
+            bt0 = std::min(bt0, b0);
             if constexpr (V == 8) CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, k_bounce<TRI, STAGE>, 128, smem));
             else CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bt, k_trace_shade_rf<V, TRI, false, STAGE>, 128, smem));
             CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, k_shadow_rf<V, TRI, STAGE>, 128, smem));
@@ -615,7 +618,8 @@ template <int V, int TRI, bool STAGE = false> void launch_depth(cwp_renderer* r,
     if (escape) k_escape<V, TRI, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
     if constexpr (V != 4) {
         if (rf && !escape) {
-            if (a.depth == 0) k_trace_shade_rf<V, TRI, true, STAGE><<<gt0, 128, sm, r->st>>>(a, r->P);
+            if (a.depth == 0 && r->O.traversal == 1) k_trace_shade_rf<V, TRI, true, STAGE><<<gt0, 128, sm, r->st>>>(a, r->P);
+            else if (a.depth == 0) k_trace_shade<V, TRI, true, STAGE><<<gt0, 128, sm, r->st>>>(a, r->P);
             else if constexpr (V == 8) k_bounce<TRI, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
             else k_trace_shade_rf<V, TRI, false, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
         }
@@ -814,8 +818,10 @@ extern "C" int cwp_renderer_init(cwp_renderer* r, const cwp_params* p, const cwp
     const int V = r->scene.variant, T = r->scene.tri;
     CWPB_CHECK(o->traversal >= 0 && o->traversal <= 2, CWP_ERR_INVALID, "traversal %d is not 0, 1 or 2", o->traversal);
     CWPB_CHECK(!(o->traversal == 1 && V == 4), CWP_ERR_INVALID, "refill traversal is available for BVH2 and CWBVH, not BVH4");
-    // auto (measured on B200, 117k-triangle box field): refill pays for CWBVH closest-hit traversal; the shadow pass
-    // (coherent rays towards the sun) and BVH2 (bound by dependent node-fetch latency) run faster per 32-ray batch
+    // auto (measured on B200, 117k-triangle box field): refill pays for CWBVH bounces; camera rays (a warp's are samples of one
+    // pixel: 17.4 ms a 512x512x256 frame against 18.7 / 19.8 / 22.5 with refill at 28 / 24 / 16 idle lanes, and its shadow queue, then in
+    // whole warps, 6.8 against 7.5), the shadow pass (coherent rays towards the sun) and BVH2 (bound by dependent node-fetch
+    // latency) run faster per 32-ray batch
     r->refill = o->traversal == 1 || (o->traversal == 0 && V == 8);
     r->refillShadow = o->traversal == 1;
     // CWBVH top levels staged in shared memory: stage_levels 0 = the default, < 0 none, 1..3 levels 0..L (at most
