@@ -41,49 +41,50 @@ struct BatchArgs {
 // pushed like inner nodes (as ~instance) and entered when they come up.
 template <int V, bool ANY>
 struct TwoLevel {
-    float3 o, d; float tmin, idx, idy, idz, ox, oy, oz;
-    float hitT, hu, hv; int hitTri, hitInst;
+    // The state that both levels use (tmin, the hit's t, u, v) lives in blas alone, and the world ray's origin and direction are read
+    // again from the queue on entering an instance, beside the instance's own record: 10 registers less across the traversal
+    // (spills of the 64-register kernels 244 -> 140 bytes closest, 212 -> 156 any).
+    float idx, idy, idz, ox, oy, oz; int hitTri, hitInst;
     int next, tsp, inst, budget;
     TravState<V, ANY, 0> blas;
 
-    __device__ __forceinline__ bool begin(float3 o_, float3 d_, float tmin_, float tmax_, int troot) {
-        o = o_; d = d_; tmin = tmin_; hitT = tmax_; hu = hv = 0.f; hitTri = -1; hitInst = -1;
+    __device__ __forceinline__ bool begin(float3 o, float3 d, float tmin, float tmax, int troot) {
+        blas.tmin = tmin; blas.hitT = tmax; blas.hu = blas.hv = 0.f; hitTri = -1; hitInst = -1;
         idx = safe_rcp(d.x); idy = safe_rcp(d.y); idz = safe_rcp(d.z);
         ox = -o.x * idx; oy = -o.y * idy; oz = -o.z * idz;
         next = troot; tsp = 0; inst = -1; budget = kVisitBudget;
         return troot < 0;   // an empty scene: nothing to traverse
     }
-    // enter instance k: ray into object space, BLAS traversal from the instance's root
-    __device__ __forceinline__ void enter(const float4* __restrict__ instances, const int* __restrict__ meshRoot, int k) {
-        const float4* I = instances + 7 * (size_t)k;
+    // enter instance i: ray k of the queue into object space, BLAS traversal from the instance's root
+    __device__ __forceinline__ void enter(const BatchArgs& a, long long k, int i) {
+        const float4* I = a.inst + 7 * (size_t)i;
+        const float3 o = xyz(__ldg(a.ro + k)), d = xyz(__ldg(a.rd + k));
         const float4 r0 = ld4(I), r1 = ld4(I + 1), r2 = ld4(I + 2);
-        const int root = __ldg(meshRoot + __float_as_int(ld4(I + 6).y));
+        const int root = __ldg(a.meshRoot + __float_as_int(ld4(I + 6).y));
         const float3 lo_ = f3(r0.x * o.x + r0.y * o.y + r0.z * o.z + r0.w, r1.x * o.x + r1.y * o.y + r1.z * o.z + r1.w, r2.x * o.x + r2.y * o.y + r2.z * o.z + r2.w);
         const float3 ld_ = f3(r0.x * d.x + r0.y * d.y + r0.z * d.z, r1.x * d.x + r1.y * d.y + r1.z * d.z, r2.x * d.x + r2.y * d.y + r2.z * d.z);
-        blas.begin(lo_, ld_, tmin, hitT, root);
-        inst = k;
+        const float hu = blas.hu, hv = blas.hv;
+        blas.begin(lo_, ld_, blas.tmin, blas.hitT, root);
+        blas.hu = hu; blas.hv = hv;   // (of the hit so far)
+        inst = i;
     }
     // one BLAS node visit of the current instance (inst >= 0); on leaving the instance, its hit is merged and the next
     // TLAS entry taken. True when the ray is finished.
     template <class TS, class BS>
-    __device__ __forceinline__ bool step_blas(const BatchArgs& a, TS& tstack, BS& bstack, int& err) {
+    __device__ __forceinline__ bool step_blas(const BatchArgs& a, long long k, TS& tstack, BS& bstack, int& err) {
         if (!blas.step(a.nodes, a.tris, bstack, err)) return false;
-        if (blas.hitTri >= 0 && blas.hitT < hitT) { hitT = blas.hitT; hitTri = blas.hitTri; hu = blas.hu; hv = blas.hv; hitInst = inst; }
+        if (blas.hitTri >= 0) { hitTri = blas.hitTri; hitInst = inst; }   // (a hit there is closer than the one before)
         inst = -1;
         if (ANY && hitTri >= 0) return true;
         if (tsp == 0) return true;
         next = tstack[--tsp];
-        if (next < 0) { enter(a.inst, a.meshRoot, ~next); return false; }
+        if (next < 0) enter(a, k, ~next);
         return false;
-    }
-    template <class TS, class BS>
-    __device__ __forceinline__ bool step(const BatchArgs& a, TS& tstack, BS& bstack, int& err) {
-        return inst >= 0 ? step_blas(a, tstack, bstack, err) : step_tlas(a, tstack, err);
     }
     // one TLAS node visit (inst < 0): nearer children first, an instance entered when it comes up. True when the ray
     // is finished.
     template <class TS>
-    __device__ __forceinline__ bool step_tlas(const BatchArgs& a, TS& tstack, int& err) {
+    __device__ __forceinline__ bool step_tlas(const BatchArgs& a, long long k, TS& tstack, int& err) {
         if (--budget < 0) { err |= kTravBudget; return true; }
         if (a.tlasW == 4) {   // four children, hit ones sorted by entry distance, nearest taken, others pushed far to near
             const float INF = 3.4e38f;
@@ -97,8 +98,8 @@ struct TwoLevel {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const float x0 = fmaf(LX[j], idx, ox), x1 = fmaf(HX[j], idx, ox), y0 = fmaf(LY[j], idy, oy), y1 = fmaf(HY[j], idy, oy), z0 = fmaf(LZ[j], idz, oz), z1 = fmaf(HZ[j], idz, oz);
-                const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), tmin));
-                const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), hitT));
+                const float tn = fmaxf(fmaxf(fminf(x0, x1), fminf(y0, y1)), fmaxf(fminf(z0, z1), blas.tmin));
+                const float tf = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fminf(fmaxf(z0, z1), blas.hitT));
                 ht[j] = CC[j] >= 0 && tn <= tf ? tn : INF;
                 he[j] = KK[j] > 0 ? ~CC[j] : CC[j];
             }
@@ -114,7 +115,7 @@ struct TwoLevel {
                 if (ht[1] < INF) tstack[tsp++] = he[1];
                 go = he[0];
             }
-            if (go < 0) enter(a.inst, a.meshRoot, ~go); else next = go;
+            if (go < 0) enter(a, k, ~go); else next = go;
             return false;
         }
         const float4* nb = a.tlas + 4 * (size_t)next;
@@ -122,10 +123,10 @@ struct TwoLevel {
         const int c0 = __float_as_int(mt.x), c1 = __float_as_int(mt.y), k0 = __float_as_int(mt.z), k1 = __float_as_int(mt.w);
         const float a0 = fmaf(n0.x, idx, ox), a1 = fmaf(n0.y, idx, ox), a2 = fmaf(n0.z, idy, oy), a3 = fmaf(n0.w, idy, oy), a4 = fmaf(nz.x, idz, oz), a5 = fmaf(nz.y, idz, oz);
         const float b0 = fmaf(n1.x, idx, ox), b1 = fmaf(n1.y, idx, ox), b2 = fmaf(n1.z, idy, oy), b3 = fmaf(n1.w, idy, oy), b4 = fmaf(nz.z, idz, oz), b5 = fmaf(nz.w, idz, oz);
-        const float t0n = fmaxf(fmaxf(fminf(a0, a1), fminf(a2, a3)), fmaxf(fminf(a4, a5), tmin));
-        const float t0f = fminf(fminf(fmaxf(a0, a1), fmaxf(a2, a3)), fminf(fmaxf(a4, a5), hitT));
-        const float t1n = fmaxf(fmaxf(fminf(b0, b1), fminf(b2, b3)), fmaxf(fminf(b4, b5), tmin));
-        const float t1f = fminf(fminf(fmaxf(b0, b1), fmaxf(b2, b3)), fminf(fmaxf(b4, b5), hitT));
+        const float t0n = fmaxf(fmaxf(fminf(a0, a1), fminf(a2, a3)), fmaxf(fminf(a4, a5), blas.tmin));
+        const float t0f = fminf(fminf(fmaxf(a0, a1), fmaxf(a2, a3)), fminf(fmaxf(a4, a5), blas.hitT));
+        const float t1n = fmaxf(fmaxf(fminf(b0, b1), fminf(b2, b3)), fmaxf(fminf(b4, b5), blas.tmin));
+        const float t1f = fminf(fminf(fmaxf(b0, b1), fmaxf(b2, b3)), fminf(fmaxf(b4, b5), blas.hitT));
         const bool h0 = c0 >= 0 && t0n <= t0f, h1 = c1 >= 0 && t1n <= t1f;
         int e0 = k0 > 0 ? ~c0 : c0, e1 = k1 > 0 ? ~c1 : c1;   // entries: node >= 0, instance as ~id
         int go;
@@ -135,7 +136,7 @@ struct TwoLevel {
             tstack[tsp++] = e1; go = e0;
         } else if (h0 || h1) go = h0 ? e0 : e1;
         else { if (tsp == 0) return true; go = tstack[--tsp]; }
-        if (go < 0) enter(a.inst, a.meshRoot, ~go); else next = go;
+        if (go < 0) enter(a, k, ~go); else next = go;
         return false;
     }
 };
@@ -159,15 +160,16 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_trace(const BatchAr
     LocalStack lstack;
     SharedStack<Entry> sstack{ reinterpret_cast<Entry*>(smem) + threadIdx.x, (int)blockDim.x };
     long long k = -1; bool fin = false, drained = false;
+    const int cap = warp_share(nRays, gridDim.x * (blockDim.x >> 5));   // a queue that does not fill the GPU is spread over all warps
     for (;;) {
         if (fin) {
-            if (!ANY) a.hits[k] = make_float4(ray.hitT, ray.hu, ray.hv, __int_as_float(ray.hitTri));
-            else if (a.hits) a.hits[k] = make_float4(ray.hitT, ray.hu, ray.hv, __int_as_float(ray.hitTri));
+            if (!ANY) a.hits[k] = make_float4(ray.blas.hitT, ray.blas.hu, ray.blas.hv, __int_as_float(ray.hitTri));
+            else if (a.hits) a.hits[k] = make_float4(ray.blas.hitT, ray.blas.hu, ray.blas.hv, __int_as_float(ray.hitTri));
             a.hitInst[k] = ray.hitInst;
             k = -1; fin = false;
         }
         if (!drained) {
-            const bool need = k < 0;
+            const bool need = k < 0 && lane < cap;
             const unsigned nm = __ballot_sync(0xffffffffu, need);
             if (nm) {
                 const int leader = __ffs(nm) - 1;
@@ -177,12 +179,12 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_trace(const BatchAr
                 const long long kk = base + __popc(nm & lane_mask_lt());
                 if (need && kk < nRays) {
                     k = kk;
-                    const float4 O = __ldcs(a.ro + k), D = __ldcs(a.rd + k);
+                    const float4 O = __ldg(a.ro + k), D = __ldg(a.rd + k);
                     const int sc = __ldcs(a.sceneOf + k);
                     const int root = sc >= 0 && sc < a.nScenes ? __ldg(a.sceneRoot + sc) : -1;
                     fin = ray.begin(xyz(O), xyz(D), O.w, D.w, root);
                 }
-                drained = __any_sync(0xffffffffu, need && kk >= nRays);
+                drained = cap < 32 || __any_sync(0xffffffffu, need && kk >= nRays);
             }
         }
         if (!__any_sync(0xffffffffu, k >= 0)) break;
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_trace(const BatchAr
                 const bool doB = __popc(inB) >= 2 * __popc(inT);
                 act = act && ((ray.inst >= 0) == doB);
             }
-            if (act) fin = ray.inst >= 0 ? (SMEM ? ray.step_blas(a, tstack, sstack, e) : ray.step_blas(a, tstack, lstack, e)) : ray.step_tlas(a, tstack, e);
+            if (act) fin = ray.inst >= 0 ? (SMEM ? ray.step_blas(a, k, tstack, sstack, e) : ray.step_blas(a, k, tstack, lstack, e)) : ray.step_tlas(a, k, tstack, e);
             const unsigned busy = __ballot_sync(0xffffffffu, k >= 0 && !fin);
             if (!busy || (!drained && 32 - __popc(busy) >= a.fetch)) break;
         }
