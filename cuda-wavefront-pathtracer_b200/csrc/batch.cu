@@ -228,6 +228,7 @@ struct cwp_batch {
     float4* triV = nullptr;              // input triangles, 3 float4 each
     float4* nrm = nullptr;               // corner normals, 3 float4 per triangle in mesh order (zero for meshes without), or null
     float4 *primLo = nullptr, *primHi = nullptr, *meshBox = nullptr;
+    void *arena = nullptr, *instArena = nullptr, *sceneArena = nullptr;   // the allocations behind the mesh, instance and scene arrays
     int* meshFirstDev = nullptr;
     int* meshRoot[3] = { nullptr, nullptr, nullptr }; std::vector<int> meshRootHost[3];   // per layout width
     int builder = 0;
@@ -259,11 +260,8 @@ static void batch_free(cwp_batch* b) {
     cudaSetDevice(b->device);
     for (auto& l : b->lay) free_wide(l);
     b->blasB.release(); b->tlasB.release();
-    cudaFree(b->triV); cudaFree(b->nrm); cudaFree(b->primLo); cudaFree(b->primHi); cudaFree(b->meshBox); cudaFree(b->meshFirstDev);
-    cudaFree(b->inst); cudaFree(b->instLo); cudaFree(b->instHi); cudaFree(b->tlas); cudaFree(b->tlas4); cudaFree(b->sceneRoot); cudaFree(b->segFirstTlas);
+    cudaFree(b->arena); cudaFree(b->nrm); cudaFree(b->instArena); cudaFree(b->sceneArena);
     cudaFree(b->uInst); cudaFree(b->uLo); cudaFree(b->uHi); cudaFree(b->dstFirstTlas);
-    cudaFree(b->err); cudaFree(b->cursor);
-    for (int i = 0; i < 3; i++) cudaFree(b->meshRoot[i]);
     if (b->st) cudaStreamDestroy(b->st);
     if (b->e0) cudaEventDestroy(b->e0);
     if (b->e1) cudaEventDestroy(b->e1);
@@ -361,21 +359,60 @@ static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_
         CWPB_CHECK((int64_t)b->meshFirst[m + 1] < (1ll << 30), CWP_ERR_INVALID, "more than 2^30 triangles in one batch");
     }
     b->nTris = b->meshFirst[n];
-    // triangle soup, 3 float4 per triangle: (v0, local id), (v1, material), (v2, 0); vertex indices and coordinates checked
-    std::vector<float4> soup((size_t)3 * b->nTris);
-    for (int m = 0; m < n; m++) {
-        const cwp_mesh_view& v = meshes[m];
-        for (int64_t t = 0; t < v.n_tris; t++) {
-            float4* o = &soup[(size_t)3 * (b->meshFirst[m] + t)];
-            for (int k = 0; k < 3; k++) {
-                const int vi = v.faces[3 * t + k];
-                CWPB_CHECK(vi >= 0 && vi < v.n_verts, CWP_ERR_INVALID, "mesh %d triangle %lld: vertex index %d out of range", m, (long long)t, vi);
-                const float* p = v.verts + 3 * (size_t)vi;
-                CWPB_CHECK(std::isfinite(p[0]) && std::isfinite(p[1]) && std::isfinite(p[2]), CWP_ERR_INVALID, "mesh %d: non-finite vertex %d", m, vi);
-                o[k] = make_float4(p[0], p[1], p[2], 0.f);
-            }
-            int id = (int)t, mat = v.face_mat ? v.face_mat[t] : 0;
-            memcpy(&o[0].w, &id, 4); memcpy(&o[1].w, &mat, 4);
+    // the batch's own arrays in one allocation
+    auto place = [&](Carver c) {
+        c.take(b->triV, (size_t)3 * b->nTris); c.take(b->primLo, (size_t)b->nTris); c.take(b->primHi, (size_t)b->nTris); c.take(b->meshBox, (size_t)2 * n);
+        c.take(b->meshFirstDev, (size_t)n + 1); c.take(b->err, 1); c.take(b->cursor, 1);
+        for (int i = 0; i < 3; i++) if (b->widths & (1 << (2 << i))) c.take(b->meshRoot[i], (size_t)n);
+        return c.at;
+    };
+    CWPB_CUDA(cudaMalloc(&b->arena, place(Carver(nullptr))));
+    place(Carver(b->arena));
+    CWPB_CUDA(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking));
+    CWPB_CUDA(cudaEventCreate(&b->e0)); CWPB_CUDA(cudaEventCreate(&b->e1));
+    b->blasB.device = b->device; b->tlasB.device = b->device;
+    b->builder = opt ? opt->builder : 0;
+    if (b->builder == 0) { if (int rc = b->blasB.reserve(b->nTris, n)) return rc; }
+    // Triangle records, 3 float4 per triangle: (v0, local id), (v1, material), (v2, 0). The meshes go up as they are (half the
+    // bytes of the records) and a kernel gathers them and checks vertex indices and coordinates.
+    {
+        std::vector<RawMesh> raw(n);
+        long long words = 0;
+        for (int m = 0; m < n; m++) {
+            const cwp_mesh_view& v = meshes[m];
+            raw[m].vert = words; words += 3 * v.n_verts;
+            raw[m].face = words; words += 3 * v.n_tris;
+            raw[m].mat = v.face_mat ? words : -1; if (v.face_mat) words += v.n_tris;
+            raw[m].first = b->meshFirst[m]; raw[m].nVerts = v.n_verts;
+        }
+        unsigned* dWords = nullptr; RawMesh* dRaw = nullptr; unsigned long long* dBad = nullptr;
+        auto placeRaw = [&](Carver c) { c.take(dRaw, (size_t)n); c.take(dBad, 1); c.take(dWords, (size_t)words); return c.at; };
+        // a temporary: in the builder's node array where it fits (written only after the gather)
+        const size_t bytes = placeRaw(Carver(nullptr));
+        void* own = nullptr;
+        if (b->builder == 0 && bytes <= (size_t)64 * b->blasB.capPrims) placeRaw(Carver(b->blasB.nodes));
+        else { CWPB_CUDA(cudaMalloc(&own, bytes)); placeRaw(Carver(own)); }
+        cudaError_t e = cudaMemcpyAsync(dRaw, raw.data(), (size_t)n * sizeof(RawMesh), cudaMemcpyHostToDevice, b->st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(dBad, 0xff, sizeof(unsigned long long), b->st);
+        for (int m = 0; m < n && e == cudaSuccess; m++) {
+            const cwp_mesh_view& v = meshes[m];
+            e = cudaMemcpyAsync(dWords + raw[m].vert, v.verts, (size_t)v.n_verts * 12, cudaMemcpyHostToDevice, b->st);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(dWords + raw[m].face, v.faces, (size_t)v.n_tris * 12, cudaMemcpyHostToDevice, b->st);
+            if (e == cudaSuccess && v.face_mat) e = cudaMemcpyAsync(dWords + raw[m].mat, v.face_mat, (size_t)v.n_tris * 4, cudaMemcpyHostToDevice, b->st);
+        }
+        unsigned long long bad = ~0ull;
+        if (e == cudaSuccess) { gather_triangles(dWords, dRaw, n, b->nTris, b->triV, dBad, b->st); e = cudaGetLastError(); }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, dBad, sizeof bad, cudaMemcpyDeviceToHost, b->st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(b->meshFirstDev, b->meshFirst.data(), (size_t)(n + 1) * sizeof(int), cudaMemcpyHostToDevice, b->st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
+        cudaFree(own);
+        CWPB_CUDA(e);
+        if (bad != ~0ull) {   // the first corner that failed: which of the two checks, as the host sees it
+            int m = 0; const int64_t i = (int64_t)(bad >> 2);
+            while (m + 1 < n && b->meshFirst[m + 1] <= i) m++;
+            const int64_t t = i - b->meshFirst[m]; const int vi = meshes[m].faces[3 * t + (int)(bad & 3)];
+            CWPB_CHECK(vi >= 0 && vi < meshes[m].n_verts, CWP_ERR_INVALID, "mesh %d triangle %lld: vertex index %d out of range", m, (long long)t, vi);
+            return set_error(CWP_ERR_INVALID, "mesh %d: non-finite vertex %d", m, vi);
         }
     }
     // corner normals of the meshes that have them (shading normals of the serving integrator)
@@ -391,30 +428,17 @@ static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_
                 nr[(size_t)3 * (b->meshFirst[m] + t) + k] = make_float4(q[0], q[1], q[2], 0.f);
             }
     }
-    CWPB_CUDA(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking));
-    CWPB_CUDA(cudaEventCreate(&b->e0)); CWPB_CUDA(cudaEventCreate(&b->e1));
     if (!nr.empty()) {
         CWPB_CUDA(cudaMalloc(&b->nrm, nr.size() * sizeof(float4)));
         CWPB_CUDA(cudaMemcpy(b->nrm, nr.data(), nr.size() * sizeof(float4), cudaMemcpyHostToDevice));
     }
-    CWPB_CUDA(cudaMalloc(&b->err, sizeof(int))); CWPB_CUDA(cudaMemset(b->err, 0, sizeof(int)));
-    CWPB_CUDA(cudaMalloc(&b->cursor, sizeof(unsigned long long)));
-    CWPB_CUDA(cudaMalloc(&b->triV, soup.size() * sizeof(float4)));
-    CWPB_CUDA(cudaMalloc(&b->primLo, (size_t)b->nTris * sizeof(float4))); CWPB_CUDA(cudaMalloc(&b->primHi, (size_t)b->nTris * sizeof(float4)));
-    CWPB_CUDA(cudaMalloc(&b->meshBox, (size_t)2 * n * sizeof(float4)));
-    CWPB_CUDA(cudaMalloc(&b->meshFirstDev, (size_t)(n + 1) * sizeof(int)));
-    CWPB_CUDA(cudaMemcpyAsync(b->triV, soup.data(), soup.size() * sizeof(float4), cudaMemcpyHostToDevice, b->st));
-    CWPB_CUDA(cudaMemcpyAsync(b->meshFirstDev, b->meshFirst.data(), (size_t)(n + 1) * sizeof(int), cudaMemcpyHostToDevice, b->st));
-    b->blasB.device = b->device; b->tlasB.device = b->device;
-    b->builder = opt ? opt->builder : 0;
+    CWPB_CUDA(cudaMemset(b->err, 0, sizeof(int)));
     CWPB_CHECK(b->builder == 0 || b->builder == 1, CWP_ERR_INVALID, "builder %d is not 0 (GPU) or 1 (host)", b->builder);
     b->tlasWidth = opt && opt->tlas_width ? opt->tlas_width : 4;
     CWPB_CHECK(b->tlasWidth == 2 || b->tlasWidth == 4, CWP_ERR_INVALID, "TLAS width %d is not 2 or 4", b->tlasWidth);
     if (b->builder == 1) {
         if (int rc = host_build(b, meshes, n, opt ? opt->spatial : 0.f)) return rc;
     } else {
-        if (int rc = b->blasB.reserve(b->nTris, n)) return rc;
-        CWPB_CUDA(cudaStreamSynchronize(b->st));
         // the timed build: boxes, keys, sort, one H-PLOC launch, root boxes, layouts
         CWPB_CUDA(cudaEventRecord(b->e0, b->st));
         triangle_boxes(b->triV, b->nTris, b->primLo, b->primHi, b->st);
@@ -433,7 +457,6 @@ static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_
     }
     for (int i = 0; i < 3; i++) {
         if (b->meshRootHost[i].empty()) continue;
-        CWPB_CUDA(cudaMalloc(&b->meshRoot[i], (size_t)n * sizeof(int)));
         CWPB_CUDA(cudaMemcpy(b->meshRoot[i], b->meshRootHost[i].data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice));
     }
     for (int i = 0; i < 3; i++) {
@@ -463,6 +486,29 @@ static int check_instances(const cwp_batch* b, const cwp_instance* h, int64_t n,
     return CWP_OK;
 }
 
+// room for n instances (with their boxes and both TLAS forms) and nScenes scenes, one allocation each
+static int ensure_scene_arrays(cwp_batch* b, int64_t n, int nScenes) {
+    if (n > b->capInst) {
+        cudaFree(b->instArena); b->instArena = nullptr;
+        b->inst = nullptr; b->instLo = b->instHi = b->tlas = b->tlas4 = nullptr; b->capInst = 0;
+        auto place = [&](Carver c) {
+            c.take(b->inst, (size_t)n); c.take(b->instLo, (size_t)n); c.take(b->instHi, (size_t)n); c.take(b->tlas, (size_t)4 * n); c.take(b->tlas4, (size_t)8 * n);
+            return c.at;
+        };
+        CWPB_CUDA(cudaMalloc(&b->instArena, place(Carver(nullptr))));
+        place(Carver(b->instArena));
+        b->capInst = n;
+    }
+    if (nScenes + 1 > b->capScenes) {
+        cudaFree(b->sceneArena); b->sceneArena = nullptr; b->sceneRoot = b->segFirstTlas = nullptr; b->capScenes = 0;
+        auto place = [&](Carver c) { c.take(b->sceneRoot, (size_t)nScenes + 1); c.take(b->segFirstTlas, (size_t)nScenes + 1); return c.at; };
+        CWPB_CUDA(cudaMalloc(&b->sceneArena, place(Carver(nullptr))));
+        place(Carver(b->sceneArena));
+        b->capScenes = nScenes + 1;
+    }
+    return CWP_OK;
+}
+
 extern "C" int cwp_batch_set_scenes(cwp_batch* b, const cwp_instance* inst, int64_t n, const int32_t* first, int32_t nScenes) {
     CWPB_CHECK(b, CWP_ERR_INVALID, "batch is NULL");
     CWPB_CHECK(first && nScenes >= 1, CWP_ERR_INVALID, "no scenes");
@@ -483,21 +529,7 @@ extern "C" int cwp_batch_set_scenes(cwp_batch* b, const cwp_instance* inst, int6
     const int nSeg = (int)seg.size() - 1;
     CWPB_CHECK(nSeg <= (1 << kSegBits), CWP_ERR_INVALID, "%d non-empty scenes (limit %d)", nSeg, 1 << kSegBits);
     CWPB_CUDA(cudaSetDevice(b->device));
-    if (n > b->capInst) {
-        cudaFree(b->inst); cudaFree(b->instLo); cudaFree(b->instHi); cudaFree(b->tlas); cudaFree(b->tlas4);
-        b->inst = nullptr; b->instLo = b->instHi = b->tlas = b->tlas4 = nullptr; b->capInst = 0;
-        CWPB_CUDA(cudaMalloc(&b->inst, (size_t)n * sizeof(cwp_instance)));
-        CWPB_CUDA(cudaMalloc(&b->instLo, (size_t)n * sizeof(float4))); CWPB_CUDA(cudaMalloc(&b->instHi, (size_t)n * sizeof(float4)));
-        CWPB_CUDA(cudaMalloc(&b->tlas, (size_t)4 * n * sizeof(float4)));
-        CWPB_CUDA(cudaMalloc(&b->tlas4, (size_t)8 * n * sizeof(float4)));
-        b->capInst = n;
-    }
-    if (nScenes + 1 > b->capScenes) {
-        cudaFree(b->sceneRoot); cudaFree(b->segFirstTlas); b->sceneRoot = b->segFirstTlas = nullptr;
-        CWPB_CUDA(cudaMalloc(&b->sceneRoot, (size_t)(nScenes + 1) * sizeof(int)));
-        CWPB_CUDA(cudaMalloc(&b->segFirstTlas, (size_t)(nScenes + 1) * sizeof(int)));
-        b->capScenes = nScenes + 1;
-    }
+    if (int rc = ensure_scene_arrays(b, n, nScenes)) return rc;
     CWPB_CUDA(cudaEventRecord(b->e0, b->st));
     if (n > 0) CWPB_CUDA(cudaMemcpyAsync(b->inst, inst, (size_t)n * sizeof(cwp_instance), cudaMemcpyHostToDevice, b->st));
     CWPB_CUDA(cudaMemcpyAsync(b->sceneRoot, rootHost.data(), (size_t)nScenes * sizeof(int), cudaMemcpyHostToDevice, b->st));
@@ -524,26 +556,12 @@ extern "C" int cwp_batch_reserve_scenes(cwp_batch* b, int32_t nScenes, int32_t c
     CWPB_CUDA(cudaSetDevice(b->device));
     const int64_t n = (int64_t)nScenes * cap;
     b->nScenes = 0;   // not traceable while the arrays change
-    if (n > b->capInst) {
-        cudaFree(b->inst); cudaFree(b->instLo); cudaFree(b->instHi); cudaFree(b->tlas); cudaFree(b->tlas4);
-        b->inst = nullptr; b->instLo = b->instHi = b->tlas = b->tlas4 = nullptr; b->capInst = 0;
-        CWPB_CUDA(cudaMalloc(&b->inst, (size_t)n * sizeof(cwp_instance)));
-        CWPB_CUDA(cudaMalloc(&b->instLo, (size_t)n * sizeof(float4))); CWPB_CUDA(cudaMalloc(&b->instHi, (size_t)n * sizeof(float4)));
-        CWPB_CUDA(cudaMalloc(&b->tlas, (size_t)4 * n * sizeof(float4)));
-        CWPB_CUDA(cudaMalloc(&b->tlas4, (size_t)8 * n * sizeof(float4)));
-        b->capInst = n;
-    }
+    if (int rc = ensure_scene_arrays(b, n, nScenes)) return rc;
     if (n > b->capU) {
         cudaFree(b->uInst); cudaFree(b->uLo); cudaFree(b->uHi); b->uInst = nullptr; b->uLo = b->uHi = nullptr; b->capU = 0;
         CWPB_CUDA(cudaMalloc(&b->uInst, (size_t)n * sizeof(cwp_instance)));
         CWPB_CUDA(cudaMalloc(&b->uLo, (size_t)n * sizeof(float4))); CWPB_CUDA(cudaMalloc(&b->uHi, (size_t)n * sizeof(float4)));
         b->capU = n;
-    }
-    if (nScenes + 1 > b->capScenes) {
-        cudaFree(b->sceneRoot); cudaFree(b->segFirstTlas); b->sceneRoot = b->segFirstTlas = nullptr;
-        CWPB_CUDA(cudaMalloc(&b->sceneRoot, (size_t)(nScenes + 1) * sizeof(int)));
-        CWPB_CUDA(cudaMalloc(&b->segFirstTlas, (size_t)(nScenes + 1) * sizeof(int)));
-        b->capScenes = nScenes + 1;
     }
     if (nScenes > b->capDst) {
         cudaFree(b->dstFirstTlas); b->dstFirstTlas = nullptr;

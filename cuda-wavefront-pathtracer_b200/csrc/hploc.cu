@@ -210,29 +210,34 @@ __global__ void __launch_bounds__(kClimbBlock) k_seg_hploc(float4* nodes, int* c
 
 int SegBuilder::reserve(int64_t n, int nSeg) {
     if (n <= capPrims && nSeg <= capSegs) return CWP_OK;
-    release();
     CWPB_CHECK(n < (1ll << 30), CWP_ERR_INVALID, "%lld primitives in one build (limit 2^30)", (long long)n);
-    CWPB_CUDA(cudaSetDevice(device));
     const int64_t cap = n > capPrims ? n : capPrims; const int cs = nSeg > capSegs ? nSeg : capSegs;
-    CWPB_CUDA(cudaMalloc(&nodes, (size_t)2 * 2 * cap * sizeof(float4)));
-    CWPB_CUDA(cudaMalloc(&count, (size_t)2 * cap * sizeof(int)));
-    CWPB_CUDA(cudaMalloc(&keys, (size_t)cap * 8)); CWPB_CUDA(cudaMalloc(&keysSorted, (size_t)cap * 8));
-    CWPB_CUDA(cudaMalloc(&vals, (size_t)cap * 4)); CWPB_CUDA(cudaMalloc(&valsSorted, (size_t)cap * 4));
-    CWPB_CUDA(cudaMalloc(&clusters, (size_t)cap * 4)); CWPB_CUDA(cudaMalloc(&bounds, (size_t)cap * 4));
-    CWPB_CUDA(cudaMalloc(&segFirst, (size_t)(cs + 1) * 4)); CWPB_CUDA(cudaMalloc(&counters, (size_t)cs * 4));
-    CWPB_CUDA(cudaMalloc(&cbox, (size_t)cs * 6 * 4));
-    tmpBytes = 0;
-    CWPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmpBytes, keys, keysSorted, vals, valsSorted, (int)cap, 0, 64));
-    CWPB_CUDA(cudaMalloc(&tmp, tmpBytes > 0 ? tmpBytes : 16));
-    capPrims = cap; capSegs = cs;
+    release();
+    CWPB_CUDA(cudaSetDevice(device));
+    size_t tb = 0;
+    CWPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keysSorted, vals, valsSorted, (int)cap, 0, 64));
+    if (tb == 0) tb = 16;
+    auto place = [&](Carver c) {
+        c.take(nodes, (size_t)2 * 2 * cap); c.take(count, (size_t)2 * cap);
+        c.take(segFirst, (size_t)cs + 1); c.take(counters, (size_t)cs); c.take(cbox, (size_t)cs * 6);
+        const size_t s0 = c.at;
+        c.take(keys, (size_t)cap); c.take(keysSorted, (size_t)cap); c.take(vals, (size_t)cap); c.take(valsSorted, (size_t)cap);
+        c.take(clusters, (size_t)cap); c.take(bounds, (size_t)cap); c.take(tmp, tb);
+        scratch = keys; scratchBytes = c.at - s0;
+        return c.at;
+    };
+    const size_t bytes = place(Carver(nullptr));
+    CWPB_CUDA(cudaMalloc(&arena, bytes));
+    place(Carver(arena));
+    tmpBytes = tb; capPrims = cap; capSegs = cs;
     return CWP_OK;
 }
 
 void SegBuilder::release() {
-    if (!capPrims && !capSegs) return;
+    if (!arena) return;
     cudaSetDevice(device);
-    cudaFree(nodes); cudaFree(count); cudaFree(keys); cudaFree(keysSorted); cudaFree(vals); cudaFree(valsSorted);
-    cudaFree(clusters); cudaFree(bounds); cudaFree(segFirst); cudaFree(counters); cudaFree(cbox); cudaFree(tmp);
+    cudaFree(arena);
+    arena = scratch = nullptr; scratchBytes = 0;
     nodes = nullptr; count = nullptr; keys = keysSorted = nullptr; vals = valsSorted = nullptr; clusters = bounds = nullptr;
     segFirst = counters = nullptr; cbox = nullptr; tmp = nullptr; tmpBytes = 0; capPrims = 0; capSegs = 0;
 }

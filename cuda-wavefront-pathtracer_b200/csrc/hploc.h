@@ -36,7 +36,9 @@ struct SegBuilder {
     int* segFirst = nullptr;                  // device copy, nSeg + 1 entries
     int* counters = nullptr;                  // next internal node id per segment
     unsigned* cbox = nullptr;                 // 6 ordered-uint bounds per segment
-    void* tmp = nullptr; size_t tmpBytes = 0;
+    char* tmp = nullptr; size_t tmpBytes = 0;
+    void* arena = nullptr;                    // the one allocation of all of the above
+    void* scratch = nullptr; size_t scratchBytes = 0;   // the part of it that is free again after build() (keys to tmp)
 
     int reserve(int64_t n, int nSeg);
     // lo / hi: n boxes (device, float4 xyz); segFirst: host array of nSeg + 1 offsets. Stream-ordered. Returns CWP_OK

@@ -14,6 +14,35 @@ __device__ __forceinline__ int node_left(const float4* bn, int i) { return __flo
 __device__ __forceinline__ int node_right(const float4* bn, int i) { return __float_as_int(__ldg(bn + 2 * i + 1).w); }
 __device__ __forceinline__ float half_area3(float3 l, float3 h) { const float3 e = h - l; return e.x * e.y + e.y * e.z + e.z * e.x; }
 
+// one thread per triangle (see wide_emit.h); the vertex reads hit L2: a mesh's vertices are a few MB and each is read by six triangles
+__global__ void __launch_bounds__(256) k_gather_triangles(const unsigned* __restrict__ words, const RawMesh* __restrict__ meshes, int nMesh, int n, float4* __restrict__ triV,
+                                                          unsigned long long* bad) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int lo = 0, hi = nMesh - 1;
+    while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (__ldg(&meshes[mid].first) <= i) lo = mid; else hi = mid - 1; }
+    const RawMesh m = meshes[lo];
+    const int t = i - m.first;
+    float4 v[3];
+    for (int k = 0; k < 3; k++) {
+        const int vi = (int)__ldg(words + m.face + 3ll * t + k);
+        float3 p = f3(0.f, 0.f, 0.f);
+        bool ok = vi >= 0 && vi < m.nVerts;
+        if (ok) {
+            const unsigned* q = words + m.vert + 3ll * vi;
+            p = f3(__uint_as_float(__ldg(q)), __uint_as_float(__ldg(q + 1)), __uint_as_float(__ldg(q + 2)));
+            ok = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+        }
+        if (!ok) { p = f3(0.f, 0.f, 0.f); atomicMin(bad, 4ull * (unsigned)i + (unsigned)k); }
+        v[k] = make_float4(p.x, p.y, p.z, 0.f);
+    }
+    v[0].w = __int_as_float(t); v[1].w = __uint_as_float(m.mat >= 0 ? __ldg(words + m.mat + t) : 0u);
+    for (int k = 0; k < 3; k++) triV[3 * (size_t)i + k] = v[k];
+}
+void gather_triangles(const unsigned* words, const RawMesh* meshes, int nMesh, int64_t n, float4* triV, unsigned long long* bad, cudaStream_t st) {
+    if (n > 0) k_gather_triangles<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(words, meshes, nMesh, (int)n, triV, bad);
+}
+
 __global__ void k_tri_boxes(const float4* __restrict__ triV, int64_t n, float4* lo, float4* hi) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -114,14 +143,14 @@ __device__ __forceinline__ unsigned quant_plane(float v, float origin, float sca
 }
 
 __global__ void k_wide_emit(int W, int leafMax, const int* __restrict__ items, int nItems, int64_t levelStart, int64_t nextStart, int rootLevel,
-                            const int* __restrict__ plan, const unsigned long long* __restrict__ prefix, int64_t triCursor,
+                            const int* __restrict__ plan, const unsigned long long* __restrict__ sums, const unsigned long long* __restrict__ prefix, int64_t triCursor,
                             const float4* __restrict__ bn, const int* __restrict__ bcnt, int nBin, const float4* __restrict__ triV, int nPrim,
                             float4* wnodes, float4* wtris, int* nextItems, int* err) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nItems) return;
     const int b = items[j];
     if (b < 0 || b >= nBin) { atomicOr(err, 1); return; }   // flagged by the plan pass; the build is rejected
-    const unsigned long long p = prefix[j];
+    const unsigned long long p = prefix[j] - sums[j];   // (prefix is inclusive; the halves do not borrow: both fields only grow)
     const int innerOff = (int)(p >> 32);
     const int64_t childBase = nextStart + innerOff, triBase = triCursor + (int64_t)(p & 0xffffffffull);
     int cref[8], ccnt[8]; float3 clo[8], chi[8];
@@ -198,8 +227,9 @@ __global__ void k_wide_emit(int W, int leafMax, const int* __restrict__ items, i
 }
 
 void free_wide(WideLayout& w) {
-    cudaFree(w.nodes); cudaFree(w.tris);
-    w.nodes = nullptr; w.tris = nullptr; w.nNodes = w.capNodes = 0;
+    if (w.arena) cudaFree(w.arena);
+    else { cudaFree(w.nodes); cudaFree(w.tris); }
+    w.arena = nullptr; w.nodes = nullptr; w.tris = nullptr; w.nNodes = w.capNodes = 0;
 }
 
 int emit_wide(const SegBuilder& B, const int* segFirstHost, int nSeg, const float4* triV, int width, int leafMax, WideLayout& out, cudaStream_t st) {
@@ -210,49 +240,50 @@ int emit_wide(const SegBuilder& B, const int* segFirstHost, int nSeg, const floa
     out.width = width;
     // wide nodes: at most the binary nodes above leaf size (<= 2 n / (leafMax + 1)) plus one root per mesh
     out.capNodes = 2 * n / (leafMax + 1) + nSeg + 64;
-    CWPB_CUDA(cudaMalloc(&out.nodes, (size_t)out.capNodes * out.stride() * sizeof(float4)));
-    CWPB_CUDA(cudaMalloc(&out.tris, (size_t)3 * n * sizeof(float4)));
-    int *items = nullptr, *next = nullptr, *plan = nullptr, *err = nullptr; unsigned long long *sums = nullptr, *prefix = nullptr; void* tmp = nullptr; size_t tmpBytes = 0;
-    unsigned long long* hostTot = nullptr;
+    auto placeOut = [&](Carver c) { c.take(out.nodes, (size_t)out.capNodes * out.stride()); c.take(out.tris, (size_t)3 * n); return c.at; };
+    CWPB_CUDA(cudaMalloc(&out.arena, placeOut(Carver(nullptr))));
+    placeOut(Carver(out.arena));
+    int *items = nullptr, *next = nullptr, *plan = nullptr, *err = nullptr; unsigned long long *sums = nullptr, *prefix = nullptr; char* tmp = nullptr; size_t tmpBytes = 0;
     const int64_t capItems = out.capNodes;
     const int nBin = (int)(2 * n - nSeg);
-    auto cleanup = [&]() { cudaFree(items); cudaFree(next); cudaFree(plan); cudaFree(err); cudaFree(sums); cudaFree(prefix); cudaFree(tmp); cudaFreeHost(hostTot); };
-    cudaError_t e = cudaMalloc(&items, (size_t)capItems * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&err, sizeof(int));
-    if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMalloc(&next, (size_t)capItems * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&plan, (size_t)capItems * 8 * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&sums, (size_t)capItems * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&prefix, (size_t)capItems * 8);
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tmpBytes, sums, prefix, (int)capItems);
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, tmpBytes > 0 ? tmpBytes : 16);
-    if (e == cudaSuccess) e = cudaMallocHost(&hostTot, 2 * sizeof(unsigned long long));
-    if (e != cudaSuccess) { cleanup(); return set_error(CWP_ERR_NOMEM, "layout scratch: %s", cudaGetErrorString(e)); }
+    CWPB_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmpBytes, sums, prefix, (int)capItems));
+    auto place = [&](Carver c) {
+        c.take(items, (size_t)capItems); c.take(next, (size_t)capItems); c.take(plan, (size_t)capItems * 8); c.take(err, 1);
+        c.take(sums, (size_t)capItems); c.take(prefix, (size_t)capItems); c.take(tmp, tmpBytes > 0 ? tmpBytes : 16);
+        return c.at;
+    };
+    const size_t need = place(Carver(nullptr));
+    void* own = nullptr;   // only where the builder's scratch is too small (tiny builds, leaf size 1)
+    cudaError_t e = cudaSuccess;
+    if (need > B.scratchBytes) e = cudaMalloc(&own, need);
+    if (e != cudaSuccess) return set_error(CWP_ERR_NOMEM, "layout scratch: %s", cudaGetErrorString(e));
+    place(Carver(own ? own : B.scratch));
+    auto cleanup = [&]() { if (own) { cudaStreamSynchronize(st); cudaFree(own); } };
+    e = cudaMemsetAsync(err, 0, sizeof(int), st);
     std::vector<int> roots(nSeg);
     for (int s = 0; s < nSeg; s++) { const int f = segFirstHost[s], m = segFirstHost[s + 1] - f; roots[s] = 2 * f - s + (m > 1 ? 2 * m - 2 : 0); }
-    e = cudaMemcpyAsync(items, roots.data(), (size_t)nSeg * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(items, roots.data(), (size_t)nSeg * 4, cudaMemcpyHostToDevice, st);
     int64_t nItems = nSeg, levelStart = 0, cursor = nSeg, triCursor = 0; int rootLevel = 1;
     while (e == cudaSuccess && nItems > 0) {
         const unsigned g = (unsigned)((nItems + 127) / 128);
         k_wide_plan<<<g, 128, 0, st>>>(width, leafMax, items, (int)nItems, rootLevel, B.nodes, B.count, nBin, plan, sums, err);
         size_t tb = tmpBytes;
-        e = cub::DeviceScan::ExclusiveSum(tmp, tb, sums, prefix, (int)nItems, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hostTot, prefix + nItems - 1, 8, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hostTot + 1, sums + nItems - 1, 8, cudaMemcpyDeviceToHost, st);
+        unsigned long long tot = 0;
+        e = cub::DeviceScan::InclusiveSum(tmp, tb, sums, prefix, (int)nItems, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&tot, prefix + nItems - 1, 8, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) break;
-        const unsigned long long tot = hostTot[0] + hostTot[1];
         const int64_t nNext = (int64_t)(tot >> 32), nTri = (int64_t)(tot & 0xffffffffull);
         if (cursor + nNext > out.capNodes || triCursor + nTri > n) { cleanup(); return set_error(CWP_ERR_INVALID, "layout emission overflow (level of %lld nodes)", (long long)nItems); }
-        k_wide_emit<<<g, 128, 0, st>>>(width, leafMax, items, (int)nItems, levelStart, cursor, rootLevel, plan, prefix, triCursor, B.nodes, B.count, nBin,
+        k_wide_emit<<<g, 128, 0, st>>>(width, leafMax, items, (int)nItems, levelStart, cursor, rootLevel, plan, sums, prefix, triCursor, B.nodes, B.count, nBin,
                                        triV, (int)n, out.nodes, out.tris, next, err);
         e = cudaGetLastError();
         levelStart = cursor; cursor += nNext; triCursor += nTri; nItems = nNext; rootLevel = 0;
         int* t = items; items = next; next = t;
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     int herr = 0;
-    if (e == cudaSuccess) e = cudaMemcpy(&herr, err, sizeof(int), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cleanup();
     if (e != cudaSuccess) return set_error(CWP_ERR_CUDA, "layout emission: %s", cudaGetErrorString(e));
     CWPB_CHECK(herr == 0, CWP_ERR_INVALID, "layout emission found a broken binary tree (node or primitive reference out of range)");

@@ -9,6 +9,7 @@ namespace cwpb {
 struct WideLayout {
     int width = 0;                       // 2, 4 or 8
     float4* nodes = nullptr; int64_t nNodes = 0, capNodes = 0;
+    void* arena = nullptr;               // emit_wide: the one allocation of nodes and tris; null: each its own
     float4* tris = nullptr;              // 3 float4 per triangle, leaf order: (v0, mesh-local id), (e1, material), (e2, 0)
     int stride() const { return width == 2 ? 4 : width == 4 ? 8 : 5; }
 };
@@ -16,7 +17,7 @@ struct WideLayout {
 // Emits one layout from the binary trees of B (built over the triangles triV: 3 float4 per triangle with the
 // mesh-local id in v0.w and the material in v1.w, as int bits). Deterministic: nodes are numbered level by level in
 // the order of their parents, whatever order the H-PLOC build allocated its binary nodes in. Synchronises the stream
-// once per tree level. leafMax: triangles per leaf (<= 3 for width 8).
+// once per tree level. leafMax: triangles per leaf (<= 3 for width 8). Scratch is taken from B's (free after its build).
 int emit_wide(const SegBuilder& B, const int* segFirstHost, int nSeg, const float4* triV, int width, int leafMax, WideLayout& out,
               cudaStream_t st);
 void free_wide(WideLayout& w);
@@ -31,6 +32,13 @@ void emit_tlas(const SegBuilder& B, int nInst, const int* segFirstDev, int nSeg,
 
 // World boxes of instances (the 8 corners of their mesh's root box through the object -> world rows).
 void instance_boxes(const cwp_instance* inst, int nInst, const float4* meshBox, float4* lo, float4* hi, cudaStream_t st);
+
+// A batch's meshes as uploaded: mesh m's vertices (3 floats each) from float vert on, its faces (3 ints each) from int face on and its
+// material ids from int mat on (-1: none) in one word array; its triangles are [first, next mesh's first) of the batch.
+struct RawMesh { long long vert, face, mat, nVerts; int first; };
+// Triangle records of all meshes (triV: (v0, mesh-local id), (v1, material), (v2, 0)), vertex indices and coordinates checked:
+// *bad (preset to all ones) becomes 4 * triangle + corner of the first offending corner; its record is zero.
+void gather_triangles(const unsigned* words, const RawMesh* meshes, int nMesh, int64_t n, float4* triV, unsigned long long* bad, cudaStream_t st);
 
 // Triangle boxes (for the BLAS build) and the mesh root boxes after it.
 void triangle_boxes(const float4* triV, int64_t n, float4* lo, float4* hi, cudaStream_t st);
