@@ -540,11 +540,10 @@ extern "C" int cwp_batch_set_scenes(cwp_batch* b, const cwp_instance* inst, int6
         emit_tlas(b->tlasB, (int)n, b->segFirstTlas, nSeg, b->tlas, b->st, nullptr, b->tlas4);
     }
     CWPB_CUDA(cudaEventRecord(b->e1, b->st));
-    CWPB_CUDA(cudaEventSynchronize(b->e1));
-    float ms = 0; CWPB_CUDA(cudaEventElapsedTime(&ms, b->e0, b->e1)); b->tlasMs = ms;
     CWPB_CUDA(cudaGetLastError());
-    b->nScenes = 0;   // not traceable until the new TLAS passes its check
+    b->nScenes = 0;   // not traceable until the new TLAS passes its check (which waits for the stream)
     if (int rc = check_tlas(b->tlas, (int)n, b->segFirstTlas, nSeg, b->err, b->st, nullptr, b->tlas4)) return rc;
+    float ms = 0; CWPB_CUDA(cudaEventElapsedTime(&ms, b->e0, b->e1)); b->tlasMs = ms;
     b->nScenes = nScenes; b->nInst = n; b->sceneFirst.assign(first, first + nScenes + 1); b->fixedCap = 0;
     return CWP_OK;
 }
