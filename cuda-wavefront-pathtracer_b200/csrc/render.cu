@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(128, CWPB_TRACE_MINB) k_bounce(const __grid_co
             const bool act = k >= 0 && !fin;
             LeafSet set;
             if (act) fin = ray.template visit<true>(nodes, a.tv, stack, set, err);
-            test_leaves<TRI, false>(w.leaves, set, a.tv, ray.hitT, ray.hitTri, ray.hu, ray.hv);
+            test_leaves<TRI, false>(w.leaves, set, a.tv, ray.hitT, ray.hitTri);
             if (act && ray.node < 0) fin = true;
             const unsigned busy = __ballot_sync(0xffffffffu, k >= 0 && !fin);
             if (!busy || (drained ? __popc(busy) <= kGroupRays : 32 - __popc(busy) >= CWPB_BOUNCE_REFILL)) break;

@@ -173,19 +173,22 @@ __device__ __forceinline__ unsigned lane_lt() { unsigned m; asm("mov.u32 %0, %%l
 
 template <int V, int TRI, bool ANY>
 __global__ void __launch_bounds__(kBatchBlock, 8) k_trace_rf(const float4* __restrict__ nodes, const float4* __restrict__ tv, const float4* __restrict__ ro,
-                                                             const float4* __restrict__ rd, float4* __restrict__ hits, int* __restrict__ occ, long long n, int* fetch, int* err) {
+                                                             const float4* __restrict__ rd, float4* __restrict__ hits, int* __restrict__ occ, int n, int* fetch, int* err) {
     constexpr bool SHARE = V == 8 && !ANY;
     __shared__ WarpLeaves<true> leaves[SHARE ? kBatchBlock / 32 : 1];
     WarpLeaves<true>& ws = leaves[SHARE ? threadIdx.x >> 5 : 0];
     const int lane = threadIdx.x & 31;
     int e = 0;
     TravState<V, ANY, TRI> ray; typename TravState<V, ANY, TRI>::Stack stack;
-    long long k = -1; bool fin = false, drained = false;
+    int k = -1; bool fin = false, drained = false;
     const int cap = warp_share(n, gridDim.x * (kBatchBlock / 32));
     for (;;) {
         if (fin) {
             if (ANY) __stcs(occ + k, ray.hitTri);
-            else __stcs(hits + k, make_float4(ray.hitT, ray.hu, ray.hv, __int_as_float(ray.hitTri)));
+            else {
+                if constexpr (SHARE) { const float2 uv = ws.uv[lane]; ray.hu = uv.x; ray.hv = uv.y; }
+                __stcs(hits + k, make_float4(ray.hitT, ray.hu, ray.hv, __int_as_float(ray.hitTri)));
+            }
             k = -1; fin = false;
         }
         if (!drained) {
@@ -193,11 +196,11 @@ __global__ void __launch_bounds__(kBatchBlock, 8) k_trace_rf(const float4* __res
             const unsigned nm = __ballot_sync(0xffffffffu, need);
             if (nm) {
                 const int leader = __ffs(nm) - 1;
-                long long base = 0;
-                if (lane == leader) base = atomicAdd((unsigned long long*)fetch, (unsigned long long)__popc(nm));
+                int base = 0;
+                if (lane == leader) base = atomicAdd(fetch, __popc(nm));
                 base = __shfl_sync(0xffffffffu, base, leader);
-                const long long kk = base + __popc(nm & lane_lt());
-                if (need && kk < n) { k = kk; const float4 O = __ldcs(ro + k), D = __ldcs(rd + k); ray.begin(xyz(O), xyz(D), O.w, D.w, 0); if constexpr (SHARE) { ws.ro[lane] = O; ws.rd[lane] = D; } }
+                const int kk = base + __popc(nm & lane_lt());
+                if (need && kk < n) { k = kk; const float4 O = __ldcs(ro + k), D = __ldcs(rd + k); ray.begin(xyz(O), xyz(D), O.w, D.w, 0); if constexpr (SHARE) { ws.ro[lane] = O; ws.rd[lane] = D; ws.uv[lane] = make_float2(0.f, 0.f); } }
                 drained = cap < 32 || __any_sync(0xffffffffu, need && kk >= n);
             }
         }
@@ -205,8 +208,9 @@ __global__ void __launch_bounds__(kBatchBlock, 8) k_trace_rf(const float4* __res
         if (!held) break;
         if constexpr (V == 8) {
             if (drained && __popc(held) <= kGroupRays) {
-                if constexpr (SHARE) ray.d = xyz(ws.rd[lane]);   // (kept in shared memory alone until here)
+                if constexpr (SHARE) { ray.d = xyz(ws.rd[lane]); const float2 uv = ws.uv[lane]; ray.hu = uv.x; ray.hv = uv.y; }   // (in shared memory alone until here)
                 finish_groups(ray, held, k, fin, nodes, tv, stack, e);
+                if constexpr (SHARE) { if (fin) ws.uv[lane] = make_float2(ray.hu, ray.hv); }
                 continue;
             }
         }
@@ -215,7 +219,7 @@ __global__ void __launch_bounds__(kBatchBlock, 8) k_trace_rf(const float4* __res
                 const bool act = k >= 0 && !fin;
                 LeafSet set;
                 if (act) fin = ray.template visit<true>(nodes, tv, stack, set, e);
-                test_leaves<TRI, true>(ws, set, tv, ray.hitT, ray.hitTri, ray.hu, ray.hv);
+                test_leaves<TRI, true>(ws, set, tv, ray.hitT, ray.hitTri);
                 if (act && ray.node < 0) fin = true;
             } else if (k >= 0 && !fin) fin = ray.step(nodes, tv, stack, e);
             const unsigned busy = __ballot_sync(0xffffffffu, k >= 0 && !fin);
@@ -319,17 +323,21 @@ template <bool ANY>
 static int launch_batch(const DeviceScene& s, const float4* o, const float4* d, void* out, long long n, int* err, cudaStream_t st, int* fetch, int refillGrid) {
     if (n <= 0) return CWP_OK;
     const float4* tv0 = s.leafData();
-    if (fetch && s.variant != 4) {   // persistent refill kernels (BVH2, CWBVH, precision form)
-        CWPB_CUDA(cudaMemsetAsync(fetch, 0, sizeof(unsigned long long), st));
-#define CWPB_R(VV, TT) k_trace_rf<VV, TT, ANY><<<refillGrid, kBatchBlock, 0, st>>>(s.nodes, tv0, o, d, (float4*)out, (int*)out, n, fetch, err)
-        if (s.precise) {   // closest hits share their triangle tests over the warp; any-hit rays keep their own
-            if (ANY) CWPB_R(16, 1);
-            else k_trace_prec_rf<<<refillGrid, kBatchBlock, 0, st>>>(s.nodes, tv0, o, d, (float4*)out, n, fetch, err);
-        }
-        else if (s.variant == 2) { if (s.tri) CWPB_R(2, 1); else CWPB_R(2, 0); }
-        else { if (s.tri) CWPB_R(8, 1); else CWPB_R(8, 0); }
+    if (fetch && s.variant != 4) {   // persistent refill kernels (BVH2, CWBVH, precision form); their ray indices are ints
+        for (long long at = 0; at < n; at += 1ll << 30) {
+            const int m = (int)std::min<long long>(n - at, 1ll << 30);
+            float4* const hits = ANY ? nullptr : (float4*)out + at; int* const occ = ANY ? (int*)out + at : nullptr;
+            CWPB_CUDA(cudaMemsetAsync(fetch, 0, sizeof(unsigned long long), st));
+#define CWPB_R(VV, TT) k_trace_rf<VV, TT, ANY><<<refillGrid, kBatchBlock, 0, st>>>(s.nodes, tv0, o + at, d + at, hits, occ, m, fetch, err)
+            if (s.precise) {   // closest hits share their triangle tests over the warp; any-hit rays keep their own
+                if (ANY) CWPB_R(16, 1);
+                else k_trace_prec_rf<<<refillGrid, kBatchBlock, 0, st>>>(s.nodes, tv0, o + at, d + at, hits, m, fetch, err);
+            }
+            else if (s.variant == 2) { if (s.tri) CWPB_R(2, 1); else CWPB_R(2, 0); }
+            else { if (s.tri) CWPB_R(8, 1); else CWPB_R(8, 0); }
 #undef CWPB_R
-        CWPB_CUDA(cudaGetLastError());
+            CWPB_CUDA(cudaGetLastError());
+        }
         return CWP_OK;
     }
     const unsigned grid = (unsigned)((n + kBatchBlock - 1) / kBatchBlock);

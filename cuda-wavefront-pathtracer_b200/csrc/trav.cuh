@@ -240,19 +240,22 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __
 // and stop at the first hit: for them the sharing measured no gain (434 vs 438 us) and their lanes test alone.
 struct LeafSet { unsigned hit = 0, m0 = 0, m1 = 0; int triBase = 0; };   // slots hit, the node's meta words, its first triangle
 template <bool UV>
-struct WarpLeaves {   // UV: hits with their barycentrics
+struct WarpLeaves {   // UV: the rays' barycentrics are kept too
     typedef typename std::conditional<UV, float4, float2>::type Hit;
-    uint2 list[32];   // first triangle and owner of the leaf that starts at this position of the round
-    Hit res[32];      // (t, triangle) or (t, triangle, u, v) of the lanes whose test hit
+    union {
+        uint2 list[32];   // first triangle and owner of the leaf that starts at this position of the round
+        Hit res[32];      // then (t, triangle) or (t, triangle, u, v) of the lanes whose test hit
+    };
     float4 ro[32];    // each lane's ray: origin, tmin; direction, current hit distance
     float4 rd[32];
+    float2 uv[UV ? 32 : 1];   // and its hit's barycentrics (here, and not in registers: they are needed again only when the ray is done)
 };
 __device__ __forceinline__ unsigned nibble_bytes(unsigned h) { return ((h * 0x00204081u) & 0x01010101u) * 255u; }   // bit i -> byte i full
 
 // All 32 lanes call it. Each ray gets the hit that testing its own triangles in slot order gives: the tests run against the
 // interval the ray had before the round, and the owner takes its hits in list order, a later one only when strictly closer.
 template <int TRI, bool UV>
-__device__ __forceinline__ void test_leaves(WarpLeaves<UV>& ws, const LeafSet& L, const float4* __restrict__ tv, float& hitT, int& hitTri, float& hu, float& hv) {
+__device__ __forceinline__ void test_leaves(WarpLeaves<UV>& ws, const LeafSet& L, const float4* __restrict__ tv, float& hitT, int& hitTri) {
     const unsigned all = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     // triangles of this lane's leaves: the count fields (meta bits 5, 6) of the hit slots, summed by a multiply
@@ -274,23 +277,23 @@ __device__ __forceinline__ void test_leaves(WarpLeaves<UV>& ws, const LeafSet& L
         }
         starts = __reduce_or_sync(all, starts);
         __syncwarp();
-        bool hit = false;
+        float t = 0.f, u = 0.f, v = 0.f; int tri = -1;
         if (base + lane < total) {
             const int at = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));   // the leaf this position belongs to
             const uint2 e = ws.list[at];
             const float4 O = ws.ro[e.y], D = ws.rd[e.y];
-            float t = D.w, u = 0.f, v = 0.f; int tri = -1;
+            t = D.w;
             leaf_hit<false, TRI>(tv, (int)e.x + lane - at, 1, xyz(O), xyz(D), O.w, t, tri, u, v);
-            hit = tri >= 0;
-            if (hit) { if constexpr (UV) ws.res[lane] = make_float4(t, __int_as_float(tri), u, v); else ws.res[lane] = make_float2(t, __int_as_float(tri)); }
         }
-        const unsigned hits = __ballot_sync(all, hit);
+        const unsigned hits = __ballot_sync(all, tri >= 0);
         if (hits) {
+            __syncwarp();   // every list entry is read before the hits take its place
+            if (tri >= 0) { if constexpr (UV) ws.res[lane] = make_float4(t, __int_as_float(tri), u, v); else ws.res[lane] = make_float2(t, __int_as_float(tri)); }
             __syncwarp();
             const int lo = max(p0 - base, 0), hi = min(incl - base, 32);
             for (unsigned mine = hi > lo ? hits & ((0xffffffffu >> (32 - (hi - lo))) << lo) : 0u; mine; mine &= mine - 1) {
                 const auto r = ws.res[__ffs(mine) - 1];
-                if (r.x < hitT) { hitT = r.x; hitTri = __float_as_int(r.y); ws.rd[lane].w = r.x; if constexpr (UV) { hu = r.z; hv = r.w; } }
+                if (r.x < hitT) { hitT = r.x; hitTri = __float_as_int(r.y); ws.rd[lane].w = r.x; if constexpr (UV) ws.uv[lane] = make_float2(r.z, r.w); }
             }
         }
         __syncwarp();
