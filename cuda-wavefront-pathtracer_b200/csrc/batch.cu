@@ -228,7 +228,7 @@ struct cwp_batch {
     float4* triV = nullptr;              // input triangles, 3 float4 each
     float4* nrm = nullptr;               // corner normals, 3 float4 per triangle in mesh order (zero for meshes without), or null
     float4 *primLo = nullptr, *primHi = nullptr, *meshBox = nullptr;
-    void *arena = nullptr, *instArena = nullptr, *sceneArena = nullptr;   // the allocations behind the mesh, instance and scene arrays
+    void* arena = nullptr;               // the allocation behind the mesh arrays
     int* meshFirstDev = nullptr;
     int* meshRoot[3] = { nullptr, nullptr, nullptr }; std::vector<int> meshRootHost[3];   // per layout width
     int builder = 0;
@@ -247,7 +247,7 @@ struct cwp_batch {
     int* dstFirstTlas = nullptr; int capDst = 0;
     // launch
     cwp_batch_tuning tuning{};
-    int* err = nullptr; unsigned long long* cursor = nullptr;
+    int* err = nullptr; unsigned long long* cursor = nullptr;   // cursor[1]: of launches beside another one (batch_trace_dev)
     cudaStream_t st = nullptr; cudaEvent_t e0 = nullptr, e1 = nullptr;
     double blasMs = 0, tlasMs = 0; int nSm = 0;
     int64_t refs[3] = { 0, 0, 0 };   // triangle records per layout (host build with spatial splits: more than nTris)
@@ -260,7 +260,8 @@ static void batch_free(cwp_batch* b) {
     cudaSetDevice(b->device);
     for (auto& l : b->lay) free_wide(l);
     b->blasB.release(); b->tlasB.release();
-    cudaFree(b->arena); cudaFree(b->nrm); cudaFree(b->instArena); cudaFree(b->sceneArena);
+    cudaFree(b->arena); cudaFree(b->nrm);
+    cudaFree(b->inst); cudaFree(b->instLo); cudaFree(b->instHi); cudaFree(b->tlas); cudaFree(b->tlas4); cudaFree(b->sceneRoot); cudaFree(b->segFirstTlas);
     cudaFree(b->uInst); cudaFree(b->uLo); cudaFree(b->uHi); cudaFree(b->dstFirstTlas);
     if (b->st) cudaStreamDestroy(b->st);
     if (b->e0) cudaEventDestroy(b->e0);
@@ -362,7 +363,7 @@ static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_
     // the batch's own arrays in one allocation
     auto place = [&](Carver c) {
         c.take(b->triV, (size_t)3 * b->nTris); c.take(b->primLo, (size_t)b->nTris); c.take(b->primHi, (size_t)b->nTris); c.take(b->meshBox, (size_t)2 * n);
-        c.take(b->meshFirstDev, (size_t)n + 1); c.take(b->err, 1); c.take(b->cursor, 1);
+        c.take(b->meshFirstDev, (size_t)n + 1); c.take(b->err, 1); c.take(b->cursor, 2);
         for (int i = 0; i < 3; i++) if (b->widths & (1 << (2 << i))) c.take(b->meshRoot[i], (size_t)n);
         return c.at;
     };
@@ -486,24 +487,22 @@ static int check_instances(const cwp_batch* b, const cwp_instance* h, int64_t n,
     return CWP_OK;
 }
 
-// room for n instances (with their boxes and both TLAS forms) and nScenes scenes, one allocation each
+// room for n instances with their boxes and both TLAS forms, and nScenes scenes (separate allocations: of a few thousand instances each
+// stays under the size from which the driver maps an allocation by itself; as one, a first TLAS took 0.1 to 0.3 ms longer)
 static int ensure_scene_arrays(cwp_batch* b, int64_t n, int nScenes) {
     if (n > b->capInst) {
-        cudaFree(b->instArena); b->instArena = nullptr;
+        cudaFree(b->inst); cudaFree(b->instLo); cudaFree(b->instHi); cudaFree(b->tlas); cudaFree(b->tlas4);
         b->inst = nullptr; b->instLo = b->instHi = b->tlas = b->tlas4 = nullptr; b->capInst = 0;
-        auto place = [&](Carver c) {
-            c.take(b->inst, (size_t)n); c.take(b->instLo, (size_t)n); c.take(b->instHi, (size_t)n); c.take(b->tlas, (size_t)4 * n); c.take(b->tlas4, (size_t)8 * n);
-            return c.at;
-        };
-        CWPB_CUDA(cudaMalloc(&b->instArena, place(Carver(nullptr))));
-        place(Carver(b->instArena));
+        CWPB_CUDA(cudaMalloc(&b->inst, (size_t)n * sizeof(cwp_instance)));
+        CWPB_CUDA(cudaMalloc(&b->instLo, (size_t)n * sizeof(float4))); CWPB_CUDA(cudaMalloc(&b->instHi, (size_t)n * sizeof(float4)));
+        CWPB_CUDA(cudaMalloc(&b->tlas, (size_t)4 * n * sizeof(float4)));
+        CWPB_CUDA(cudaMalloc(&b->tlas4, (size_t)8 * n * sizeof(float4)));
         b->capInst = n;
     }
     if (nScenes + 1 > b->capScenes) {
-        cudaFree(b->sceneArena); b->sceneArena = nullptr; b->sceneRoot = b->segFirstTlas = nullptr; b->capScenes = 0;
-        auto place = [&](Carver c) { c.take(b->sceneRoot, (size_t)nScenes + 1); c.take(b->segFirstTlas, (size_t)nScenes + 1); return c.at; };
-        CWPB_CUDA(cudaMalloc(&b->sceneArena, place(Carver(nullptr))));
-        place(Carver(b->sceneArena));
+        cudaFree(b->sceneRoot); cudaFree(b->segFirstTlas); b->sceneRoot = b->segFirstTlas = nullptr; b->capScenes = 0;
+        CWPB_CUDA(cudaMalloc(&b->sceneRoot, (size_t)(nScenes + 1) * sizeof(int)));
+        CWPB_CUDA(cudaMalloc(&b->segFirstTlas, (size_t)(nScenes + 1) * sizeof(int)));
         b->capScenes = nScenes + 1;
     }
     return CWP_OK;
@@ -633,7 +632,8 @@ extern "C" int cwp_batch_update_scenes(cwp_batch* b, const int32_t* scenes, int3
 }
 
 static int launch(cwp_batch* b, const cwp_batch_tuning& t, bool any, const float* o, const float* d, const int* sc, float* hits, int* hinst, int64_t n, cudaStream_t st,
-                  const int* nDev = nullptr) {
+                  const int* nDev = nullptr, bool side = false) {
+    unsigned long long* const cursor = b->cursor + (side ? 1 : 0);
     const WideLayout& L = b->lay[lay_index(t.width)];
     CWPB_CHECK(L.nodes, CWP_ERR_STATE, "layout width %d was not emitted (cwp_batch_options.widths)", t.width);
     BatchArgs a;
@@ -641,14 +641,14 @@ static int launch(cwp_batch* b, const cwp_batch_tuning& t, bool any, const float
     a.sceneRoot = b->sceneRoot; a.inst = reinterpret_cast<const float4*>(b->inst);
     a.meshRoot = b->meshRoot[lay_index(t.width)];
     a.nScenes = b->nScenes; a.ro = (const float4*)o; a.rd = (const float4*)d; a.sceneOf = sc; a.hits = (float4*)hits; a.hitInst = hinst;
-    a.n = n; a.nDev = nDev; a.cursor = b->cursor; a.fetch = t.fetch; a.err = b->err;
+    a.n = n; a.nDev = nDev; a.cursor = cursor; a.fetch = t.fetch; a.err = b->err;
     BatchKernel k = pick_kernel(t.width, any, t.smem_stack != 0);
     const size_t sm = t.smem_stack ? smem_bytes(t.width, t.block) : 0;
     if (sm > 48 * 1024) CWPB_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     int per = 0;
     CWPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, t.block, sm));
     CWPB_CHECK(per > 0, CWP_ERR_INVALID, "tuning (block %d, width %d, shared stack %d) does not fit an SM", t.block, t.width, t.smem_stack);
-    CWPB_CUDA(cudaMemsetAsync(b->cursor, 0, sizeof(unsigned long long), st));
+    CWPB_CUDA(cudaMemsetAsync(cursor, 0, sizeof(unsigned long long), st));
     k<<<per * b->nSm, t.block, sm, st>>>(a);
     CWPB_CUDA(cudaGetLastError());
     return CWP_OK;
@@ -787,10 +787,10 @@ extern "C" int cwp_batch_download_tlas(const cwp_batch* b, float* nodes, int64_t
 }
 
 namespace cwpb {
-int batch_trace_dev(cwp_batch* b, bool any, const float4* o, const float4* d, const int* sc, float4* hits, int* inst, int64_t n, cudaStream_t st, const int* nDev) {
+int batch_trace_dev(cwp_batch* b, bool any, const float4* o, const float4* d, const int* sc, float4* hits, int* inst, int64_t n, cudaStream_t st, const int* nDev, bool side) {
     CWPB_CHECK(b->nScenes > 0, CWP_ERR_STATE, "no scenes");
     if (n <= 0 && !nDev) return CWP_OK;
-    return launch(b, b->tuning, any, (const float*)o, (const float*)d, sc, (float*)hits, inst, n, st, nDev);
+    return launch(b, b->tuning, any, (const float*)o, (const float*)d, sc, (float*)hits, inst, n, st, nDev, side);
 }
 const float4* batch_tris(const cwp_batch* b) { return b->lay[lay_index(b->tuning.width)].tris; }
 const cwp_instance* batch_instances(const cwp_batch* b) { return b->inst; }

@@ -274,6 +274,8 @@ __global__ void __launch_bounds__(kClimbBlock) k_seg_hploc(float4* nodes, int* c
     }
 }
 
+static constexpr size_t kOneBlock = 4 << 20;   // bytes
+
 int SegBuilder::reserve(int64_t n, int nSeg) {
     if (n <= capPrims && nSeg <= capSegs) return CWP_OK;
     CWPB_CHECK(n < (1ll << 30), CWP_ERR_INVALID, "%lld primitives in one build (limit 2^30)", (long long)n);
@@ -283,27 +285,40 @@ int SegBuilder::reserve(int64_t n, int nSeg) {
     size_t tb = 0;
     CWPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keysSorted, vals, valsSorted, (int)cap, 0, 64));
     if (tb == 0) tb = 16;
-    auto place = [&](Carver c) {
-        c.take(nodes, (size_t)2 * 2 * cap); c.take(count, (size_t)2 * cap);
-        c.take(segFirst, (size_t)cs + 1); c.take(counters, (size_t)cs); c.take(cbox, (size_t)cs * 6);
-        const size_t s0 = c.at;
-        c.take(keys, (size_t)cap); c.take(keysSorted, (size_t)cap); c.take(vals, (size_t)cap); c.take(valsSorted, (size_t)cap);
-        c.take(clusters, (size_t)cap); c.take(bounds, (size_t)cap); c.take(tmp, tb);
-        scratch = keys; scratchBytes = c.at - s0;
-        return c.at;
+    // Four blocks: nodes, counts, segment arrays, scratch. In one allocation when they are large; a small build (a scene's TLAS) keeps them
+    // apart, each below the size from which the driver maps and unmaps an allocation by itself, so that the next build gets
+    // them back at once (a first TLAS of 7,864 instances after another was freed: 1.05 ms as one allocation, 0.34 as blocks)
+    auto place = [&](Carver (&c)[4]) {
+        c[0].take(nodes, (size_t)2 * 2 * cap); c[1].take(count, (size_t)2 * cap);
+        c[2].take(segFirst, (size_t)cs + 1); c[2].take(counters, (size_t)cs); c[2].take(cbox, (size_t)cs * 6);
+        c[3].take(keys, (size_t)cap); c[3].take(keysSorted, (size_t)cap); c[3].take(vals, (size_t)cap); c[3].take(valsSorted, (size_t)cap);
+        c[3].take(clusters, (size_t)cap); c[3].take(bounds, (size_t)cap); c[3].take(tmp, tb);
     };
-    const size_t bytes = place(Carver(nullptr));
-    CWPB_CUDA(cudaMalloc(&arena, bytes));
-    place(Carver(arena));
+    Carver size[4] = { Carver(nullptr), Carver(nullptr), Carver(nullptr), Carver(nullptr) };
+    place(size);
+    const size_t total = size[0].at + size[1].at + size[2].at + size[3].at;
+    char* at[4];
+    if (total > kOneBlock) {
+        CWPB_CUDA(cudaMalloc(&block[0], total));
+        at[0] = static_cast<char*>(block[0]);
+        for (int i = 1; i < 4; i++) at[i] = at[i - 1] + size[i - 1].at;
+    } else for (int i = 0; i < 4; i++) {
+        const cudaError_t e = cudaMalloc(&block[i], size[i].at);
+        if (e != cudaSuccess) { release(); CWPB_CUDA(e); }
+        at[i] = static_cast<char*>(block[i]);
+    }
+    Carver real[4] = { Carver(at[0]), Carver(at[1]), Carver(at[2]), Carver(at[3]) };
+    place(real);
+    scratch = keys; scratchBytes = size[3].at;
     tmpBytes = tb; capPrims = cap; capSegs = cs;
     return CWP_OK;
 }
 
 void SegBuilder::release() {
-    if (!arena) return;
+    if (!block[0]) return;
     cudaSetDevice(device);
-    cudaFree(arena);
-    arena = scratch = nullptr; scratchBytes = 0;
+    for (void*& p : block) { cudaFree(p); p = nullptr; }
+    scratch = nullptr; scratchBytes = 0;
     nodes = nullptr; count = nullptr; keys = keysSorted = nullptr; vals = valsSorted = nullptr; clusters = bounds = nullptr;
     segFirst = counters = nullptr; cbox = nullptr; tmp = nullptr; tmpBytes = 0; capPrims = 0; capSegs = 0;
 }

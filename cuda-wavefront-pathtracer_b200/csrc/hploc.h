@@ -37,8 +37,8 @@ struct SegBuilder {
     int* counters = nullptr;                  // next internal node id per segment
     unsigned* cbox = nullptr;                 // 6 ordered-uint bounds per segment
     char* tmp = nullptr; size_t tmpBytes = 0;
-    void* arena = nullptr;                    // the one allocation of all of the above
-    void* scratch = nullptr; size_t scratchBytes = 0;   // the part of it that is free again after build() (keys to tmp)
+    void* block[4] = { nullptr, nullptr, nullptr, nullptr };   // the allocations behind them (one for a large build)
+    void* scratch = nullptr; size_t scratchBytes = 0;   // the part that is free again after build() (keys to tmp)
 
     int reserve(int64_t n, int nSeg);
     // lo / hi: n boxes (device, float4 xyz); segFirst: host array of nSeg + 1 offsets. Stream-ordered. Returns CWP_OK

@@ -482,7 +482,12 @@ struct cwp_server {
     cudaTextureObject_t* dTexObj = nullptr; cwp_material_textures* dMtex = nullptr; int nMtex = 0; float4* dUvs = nullptr; float4* dTans = nullptr;
     SlotParams* dSlots = nullptr; int* slotCnt = nullptr; std::vector<int> hSlotCnt;
     float* ftab = nullptr;   // Blackman-Harris pixel-filter inverse CDF (CWP_FILTER_TABLE + 1 floats)
-    RayQueue q[2]{}; RayQueue qs{}; int* slotBins = nullptr; ShadowQueue sq{}; float4* hits = nullptr; int* hinst = nullptr; int* occ = nullptr; int* cnt = nullptr; int4* dChunks = nullptr;
+    RayQueue q[2]{}; RayQueue qs{}; int* slotBins = nullptr; float4* hits = nullptr; int* hinst = nullptr; int4* dChunks = nullptr;
+    // Shadow rays beside the next step: a step's any-hit launch and accumulation run on st2 while the host takes the step's counts
+    // and the next step's closest hits are traced, so queue, results and counts alternate between two sets (one without memory for two)
+    ShadowQueue sq[2]{}; int* occ[2] = { nullptr, nullptr }; int* cnt[2] = { nullptr, nullptr }; bool beside = false; int par = 0;
+    cudaStream_t st2 = nullptr; cudaEvent_t shaded = nullptr, evS[2][3] = {};   // per set: shadow start, accumulation start, end
+    bool shadowTimed[2] = { true, true };   // the set's last times are in info (false: to be taken once its end has passed)
     int* hcnt = nullptr;   // pinned: [0..1] counts, then slot counters
     SlotParams* hSlots = nullptr; int4* hChunks = nullptr; bool slotsDirty = false;   // pinned mirrors of dSlots and dChunks
     cudaMemPool_t pool = nullptr;   // request images: freed memory stays in the pool for the next admissions
@@ -494,7 +499,7 @@ struct cwp_server {
     cudaStream_t cst = nullptr;   // result copies: completed images, read while the next step runs
     std::chrono::steady_clock::time_point t0;
     std::vector<void*> allocs;
-    cudaEvent_t ev[6] = {};   // raygen start, closest start, shade start, shadow start, shadow end, accumulation start
+    cudaEvent_t ev[4] = {};   // raygen start, closest start, shade start, shade end
     cwp_server_info info{};
     bool overlap = true;        // a step returns with its launches queued; the next call takes its results
     bool inflight = false; int64_t inflightN = 0; double inflightStart = 0;   // the queued step: rays traced, host start time
@@ -542,6 +547,7 @@ extern "C" void cwp_server_destroy(cwp_server* s) {
     if (!s) return;
     cudaSetDevice(s->device);
     if (s->st) cudaStreamSynchronize(s->st);   // a queued step included
+    if (s->st2) cudaStreamSynchronize(s->st2);
     if (s->cst) cudaStreamSynchronize(s->cst);
     for (auto& kv : s->reqs) {
         if (kv.second.accum) cudaFreeAsync(kv.second.accum, s->st);
@@ -557,7 +563,10 @@ extern "C" void cwp_server_destroy(cwp_server* s) {
     if (s->hSlots) cudaFreeHost(s->hSlots);
     if (s->hChunks) cudaFreeHost(s->hChunks);
     for (cudaEvent_t e : s->ev) if (e) cudaEventDestroy(e);
+    for (auto& set : s->evS) for (cudaEvent_t e : set) if (e) cudaEventDestroy(e);
+    if (s->shaded) cudaEventDestroy(s->shaded);
     if (s->st) cudaStreamDestroy(s->st);
+    if (s->st2) cudaStreamDestroy(s->st2);
     if (s->cst) cudaStreamDestroy(s->cst);
     delete s;
 }
@@ -582,7 +591,10 @@ static int server_create(cwp_batch* b, const cwp_material* mats, int n, const in
     CWPB_CUDA(cudaSetDevice(s->device));
     CWPB_CUDA(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
     CWPB_CUDA(cudaStreamCreateWithFlags(&s->cst, cudaStreamNonBlocking));
+    CWPB_CUDA(cudaStreamCreateWithFlags(&s->st2, cudaStreamNonBlocking));
     for (cudaEvent_t& e : s->ev) CWPB_CUDA(cudaEventCreate(&e));
+    for (auto& set : s->evS) for (cudaEvent_t& e : set) CWPB_CUDA(cudaEventCreate(&e));
+    CWPB_CUDA(cudaEventCreateWithFlags(&s->shaded, cudaEventDisableTiming));
     auto alloc = [&](void** p, size_t bytes) -> int { CWPB_CUDA(cudaMalloc(p, bytes)); s->allocs.push_back(*p); return CWP_OK; };
     const size_t P = (size_t)s->O.max_paths, R = (size_t)s->O.max_requests;
     int rc = alloc((void**)&s->mats, (size_t)n * sizeof(cwp_material));
@@ -594,10 +606,12 @@ static int server_create(cwp_batch* b, const cwp_material* mats, int n, const in
     if (!rc) { rc = alloc((void**)&s->qs.o, P * 16); if (!rc) rc = alloc((void**)&s->qs.d, P * 16); if (!rc) rc = alloc((void**)&s->qs.sc, P * 4);
                if (!rc) rc = alloc((void**)&s->qs.T, P * 16); if (!rc) rc = alloc((void**)&s->qs.info, P * 16); }
     if (!rc) rc = alloc((void**)&s->slotBins, 2 * R * sizeof(int));
-    if (!rc) rc = alloc((void**)&s->sq.o, P * 16); if (!rc) rc = alloc((void**)&s->sq.d, P * 16); if (!rc) rc = alloc((void**)&s->sq.sc, P * 4);
-    if (!rc) rc = alloc((void**)&s->sq.c, P * 16);
-    if (!rc) rc = alloc((void**)&s->hits, P * 16); if (!rc) rc = alloc((void**)&s->hinst, P * 4); if (!rc) rc = alloc((void**)&s->occ, P * 4);
-    if (!rc) rc = alloc((void**)&s->cnt, 4 * sizeof(int));
+    auto placeShadow = [&](int k, Carver c) { c.take(s->sq[k].o, P); c.take(s->sq[k].d, P); c.take(s->sq[k].c, P); c.take(s->sq[k].sc, P); c.take(s->occ[k], P); c.take(s->cnt[k], 4); return c.at; };
+    void* shadowMem = nullptr;
+    const size_t shadowBytes = placeShadow(0, Carver(nullptr));
+    if (!rc) rc = alloc(&shadowMem, shadowBytes);
+    if (!rc) placeShadow(0, Carver(shadowMem));
+    if (!rc) rc = alloc((void**)&s->hits, P * 16); if (!rc) rc = alloc((void**)&s->hinst, P * 4);
     if (!rc) rc = alloc((void**)&s->dSlots, R * sizeof(SlotParams));
     if (!rc) rc = alloc((void**)&s->slotCnt, R * kSlotCounters * sizeof(int));
     if (!rc) rc = alloc((void**)&s->dChunks, (R + 1) * sizeof(int4));
@@ -617,6 +631,16 @@ static int server_create(cwp_batch* b, const cwp_material* mats, int n, const in
         CWPB_CUDA(cudaMemPoolCreate(&s->pool, &pp));
         uint64_t keep = UINT64_MAX;   // never hand freed images back to the driver between steps
         CWPB_CUDA(cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    // the second shadow set, where it leaves the reserve untouched
+    {
+        size_t freeB = 0, totalB = 0;
+        CWPB_CUDA(cudaMemGetInfo(&freeB, &totalB));
+        void* second = nullptr;
+        if ((int64_t)freeB - (int64_t)shadowBytes > s->O.hbm_reserve) {
+            if (cudaMalloc(&second, shadowBytes) == cudaSuccess) { s->allocs.push_back(second); placeShadow(1, Carver(second)); s->beside = true; }
+            else cudaGetLastError();
+        }
     }
     CWPB_CUDA(cudaMemcpy(s->mats, mats, (size_t)n * sizeof(cwp_material), cudaMemcpyHostToDevice));
     CWPB_CUDA(cudaMemcpy(s->meshMat, meshBase, (size_t)nMesh * sizeof(int), cudaMemcpyHostToDevice));
@@ -897,8 +921,20 @@ static int admit(cwp_server* s, bool& changed) {
     return CWP_OK;
 }
 
-// takes the results of the queued step: waits for its launches (the step's one host round trip), reads the queue
-// lengths and per-request counts, adds its timings and completes the requests whose paths have all finished
+// adds a set's shadow times to the statistics once (waits for its end)
+static int take_shadow_times(cwp_server* s, int p) {
+    if (s->shadowTimed[p]) return CWP_OK;
+    s->shadowTimed[p] = true;
+    float d = 0, e = 0;
+    CWPB_CUDA(cudaEventSynchronize(s->evS[p][2]));
+    CWPB_CUDA(cudaEventElapsedTime(&d, s->evS[p][0], s->evS[p][2])); CWPB_CUDA(cudaEventElapsedTime(&e, s->evS[p][1], s->evS[p][2]));
+    s->info.shadow_ms += d; s->info.accum_ms += e;
+    return CWP_OK;
+}
+
+// takes the results of the queued step: waits for its launches up to the shading (the step's one host round trip; its shadow rays may
+// still run), reads the queue lengths and per-request counts, adds its timings and completes the requests whose paths have all
+// finished, waiting for their last shadow contributions
 static int finish_step(cwp_server* s) {
     if (!s->inflight) return CWP_OK;
     s->inflight = false;
@@ -907,15 +943,21 @@ static int finish_step(cwp_server* s) {
     int64_t nNext = 0, nShadow = 0;
     if (n > 0) { nNext = s->hcnt[0]; nShadow = s->hcnt[1]; }
     {
-        float a = 0, b = 0, c = 0, d = 0;
+        float a = 0, b = 0, c = 0;
         CWPB_CUDA(cudaEventElapsedTime(&a, s->ev[0], s->ev[1])); CWPB_CUDA(cudaEventElapsedTime(&b, s->ev[1], s->ev[2]));
-        CWPB_CUDA(cudaEventElapsedTime(&c, s->ev[2], s->ev[3])); CWPB_CUDA(cudaEventElapsedTime(&d, s->ev[3], s->ev[4]));
-        float e = 0; CWPB_CUDA(cudaEventElapsedTime(&e, s->ev[5], s->ev[4]));
-        s->info.raygen_ms += a; s->info.closest_ms += b; s->info.shade_ms += c; s->info.shadow_ms += d; s->info.accum_ms += e;
+        CWPB_CUDA(cudaEventElapsedTime(&c, s->ev[2], s->ev[3]));
+        s->info.raygen_ms += a; s->info.closest_ms += b; s->info.shade_ms += c;
         s->info.steps++; s->info.rays += n; s->info.shadow_rays += nShadow;
     }
     if ((s->info.steps & 63) == 0 || nNext == 0) { if (int rc = cwp_batch_status(s->batch)) return rc; }   // traversal bounds: checked every 64 steps and when the queue drains
     s->cur ^= 1; s->nCur = nNext;
+    bool completes = !s->overlap;
+    for (int k = 0; k < R && !completes; k++)
+        if (s->slotReq[k] >= 0) { const ServeRequest& q = s->reqs[s->slotReq[k]]; completes = q.issued == q.total && s->hcnt[4 + kSlotCounters * k + 2] == q.total; }
+    if (completes) {   // (in the plain form of overlap -1 every step waits for all of its work)
+        CWPB_CUDA(cudaStreamSynchronize(s->st2));
+        for (int p = 0; p < 2; p++) if (int rc = take_shadow_times(s, p)) return rc;
+    }
     const double t = now_ms(s);
     for (int k = 0; k < R; k++) {
         if (s->slotReq[k] < 0) continue;
@@ -960,36 +1002,43 @@ static int launch_step(cwp_server* s) {
     CWPB_CUDA(cudaEventRecord(s->ev[1], s->st));
     CWPB_CUDA(cudaEventRecord(s->ev[2], s->st));
     CWPB_CUDA(cudaEventRecord(s->ev[3], s->st));
-    CWPB_CUDA(cudaEventRecord(s->ev[5], s->st));
+    if (s->beside) s->par ^= 1;
+    const int p = s->par;
+    const cudaStream_t ss = s->beside ? s->st2 : s->st;   // the shadow pass's stream
+    int* const cnt = s->cnt[p];
     if (n > 0) {
         if (int rc = batch_trace_dev(s->batch, false, in.o, in.d, in.sc, s->hits, s->hinst, n, s->st)) return rc;
         CWPB_CUDA(cudaEventRecord(s->ev[2], s->st));
-        CWPB_CUDA(cudaMemsetAsync(s->cnt, 0, 4 * sizeof(int), s->st));
+        if (int rc = take_shadow_times(s, p)) return rc;   // the set's step before the last: its shadow pass ended (or is waited for) before the set is written again
+        CWPB_CUDA(cudaMemsetAsync(cnt, 0, 4 * sizeof(int), s->st));
         ShadeArgs a{};
-        a.n = (int)n; a.in = in; a.out = out; a.sq = s->sq; a.hits = s->hits; a.hinst = s->hinst; a.inst = batch_instances(s->batch); a.tris = batch_tris(s->batch);
-        a.mats = s->mats; a.nMats = s->nMats; a.meshMat = s->meshMat; a.slots = s->dSlots; a.gdEnergy = s->O.gd_energy; a.cnt = s->cnt; a.slotCnt = s->slotCnt;
+        a.n = (int)n; a.in = in; a.out = out; a.sq = s->sq[p]; a.hits = s->hits; a.hinst = s->hinst; a.inst = batch_instances(s->batch); a.tris = batch_tris(s->batch);
+        a.mats = s->mats; a.nMats = s->nMats; a.meshMat = s->meshMat; a.slots = s->dSlots; a.gdEnergy = s->O.gd_energy; a.cnt = cnt; a.slotCnt = s->slotCnt;
         a.texObj = s->dTexObj; a.mtex = s->nMtex ? s->dMtex : nullptr; a.nMtex = s->nMtex; a.uvs = s->dUvs; a.tans = s->dTans; a.meshFirst = batch_mesh_first(s->batch);
         a.nrm = batch_normals(s->batch);
         const unsigned g = (unsigned)std::min<int64_t>((n + 127) / 128, 148 * 16);
         k_serve_shade<<<g, 128, 0, s->st>>>(a);
         CWPB_CUDA(cudaGetLastError());
         CWPB_CUDA(cudaEventRecord(s->ev[3], s->st));
+        if (s->beside) { CWPB_CUDA(cudaEventRecord(s->shaded, s->st)); CWPB_CUDA(cudaStreamWaitEvent(s->st2, s->shaded, 0)); }
         if (R > 1 && s->O.regroup >= 0) {   // regroup the next step's rays by request (continuous batching interleaves them)
             CWPB_CUDA(cudaMemsetAsync(s->slotBins, 0, 2 * R * sizeof(int), s->st));
-            k_slot_hist<<<148 * 4, 256, R * sizeof(int), s->st>>>(s->cnt, out.info, s->slotBins, R);
+            k_slot_hist<<<148 * 4, 256, R * sizeof(int), s->st>>>(cnt, out.info, s->slotBins, R);
             k_slot_scan<<<1, 1024, 0, s->st>>>(s->slotBins, s->slotBins + R, R);
-            k_slot_scatter<<<148 * 8, 256, 0, s->st>>>(s->cnt, out, s->qs, s->slotBins + R);
+            k_slot_scatter<<<148 * 8, 256, 0, s->st>>>(cnt, out, s->qs, s->slotBins + R);
             CWPB_CUDA(cudaGetLastError());
             std::swap(s->q[s->cur ^ 1], s->qs);   // the regrouped copy is the next step's input
         }
         // shadow rays: count on the device, no host round trip before the any-hit launch
-        if (int rc = batch_trace_dev(s->batch, true, s->sq.o, s->sq.d, s->sq.sc, nullptr, s->occ, 0, s->st, s->cnt + 1)) return rc;
-        CWPB_CUDA(cudaEventRecord(s->ev[5], s->st));
-        k_serve_shadow_accum<<<148 * 8, 256, 0, s->st>>>(s->cnt + 1, s->sq, s->occ, s->dSlots);
+        CWPB_CUDA(cudaEventRecord(s->evS[p][0], ss));
+        if (int rc = batch_trace_dev(s->batch, true, s->sq[p].o, s->sq[p].d, s->sq[p].sc, nullptr, s->occ[p], 0, ss, cnt + 1, s->beside)) return rc;
+        CWPB_CUDA(cudaEventRecord(s->evS[p][1], ss));
+        k_serve_shadow_accum<<<148 * 8, 256, 0, ss>>>(cnt + 1, s->sq[p], s->occ[p], s->dSlots);
         CWPB_CUDA(cudaGetLastError());
+        CWPB_CUDA(cudaEventRecord(s->evS[p][2], ss));
+        s->shadowTimed[p] = false;
     }
-    CWPB_CUDA(cudaEventRecord(s->ev[4], s->st));
-    if (n > 0) CWPB_CUDA(cudaMemcpyAsync(s->hcnt, s->cnt, 2 * sizeof(int), cudaMemcpyDeviceToHost, s->st));
+    if (n > 0) CWPB_CUDA(cudaMemcpyAsync(s->hcnt, cnt, 2 * sizeof(int), cudaMemcpyDeviceToHost, s->st));
     CWPB_CUDA(cudaMemcpyAsync(s->hcnt + 4, s->slotCnt, (size_t)R * kSlotCounters * sizeof(int), cudaMemcpyDeviceToHost, s->st));
     s->inflight = true; s->inflightN = n;
     return CWP_OK;
@@ -1010,6 +1059,7 @@ extern "C" int cwp_server_step(cwp_server* s, int32_t* nActive, int32_t* nPendin
     s->info.admit_ms += now_ms(s) - admitStart;
     if (changed) {
         CWPB_CUDA(cudaStreamSynchronize(s->st));
+        CWPB_CUDA(cudaStreamSynchronize(s->st2));   // (the update's check and the traversals share the batch's status word)
         const double t = now_ms(s);
         if (int rc = rebuild_tlas(s)) return rc;
         s->info.tlas_ms += now_ms(s) - t; s->info.tlas_rebuilds++;
