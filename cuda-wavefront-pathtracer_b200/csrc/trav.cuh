@@ -49,6 +49,13 @@ __device__ __forceinline__ void fetch_node(const StagedNodes& n, int node, float
 // reciprocal direction with the reference's safe epsilon (traverse.cuh:48-50)
 __device__ __forceinline__ float safe_rcp(float x) { const float eps = 1e-20f; return 1.f / (fabsf(x) > eps ? x : copysignf(eps, x)); }
 
+// a * b + c of two floats at once (one instruction on sm_100), each rounded as fmaf; and of a float4's components
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ void fma_four(float4 v, float b, float c, float (&out)[4]) {
+    const float2 b2 = make_float2(b, b), c2 = make_float2(c, c), p = fma2(make_float2(v.x, v.y), b2, c2), q = fma2(make_float2(v.z, v.w), b2, c2);
+    out[0] = p.x; out[1] = p.y; out[2] = q.x; out[3] = q.y;
+}
+
 // ---------------- leaf tests ----------------
 template <bool ANY, int TRI>
 __device__ __forceinline__ bool leaf_hit(const float4* __restrict__ tv, int first, int cnt, float3 o, float3 d, float tmin,
@@ -225,9 +232,6 @@ __device__ __forceinline__ unsigned byte_of(unsigned w, int s) { return (w >> (8
 __device__ __forceinline__ float qbyte(unsigned w, int s) {
     return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540u | (unsigned)(s & 3))) - 8388608.0f;
 }
-
-// a * b + c of two floats at once (one instruction on sm_100), each rounded as fmaf
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
 // ---- triangle tests shared over the warp (closest hits) ----
 // The rays' hit leaves of one node visit. Of a warp's 24 active rays about 9 hit a leaf per visit, of 1 to 3 triangles each:
