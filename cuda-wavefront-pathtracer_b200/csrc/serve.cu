@@ -10,7 +10,8 @@
 //   4. shading (OpenPBR-subset BSDFs, one light sample per vertex over the sun, the emissive triangles and an
 //      environment map, MIS with BSDF sampling, Russian roulette): continuations into the next queue, shadow rays into
 //      the shadow queue, per-slot counts of traced, shadow and finished paths;
-//   5. one any-hit launch over the shadow queue and the accumulation of the unoccluded contributions;
+//   5. one any-hit launch over the shadow queue and the accumulation of the unoccluded contributions, on a second stream
+//      beside the next step (where device memory allows a second shadow set);
 //   6. completion: a request whose paths were all issued and have all finished is done.
 // A request's image depends only on its own inputs: every random number is keyed by (pixel, sample, depth, dimension,
 // request seed), and shading reads only its own slot's parameters. max_requests = 1 gives the plain form (one request

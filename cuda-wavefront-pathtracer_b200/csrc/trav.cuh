@@ -325,7 +325,7 @@ struct CwbvhTrav {
     // One node visit. SHARE = false: the hit leaves are tested here; true when the ray is finished. SHARE = true: they are
     // returned in `leaves` for test_leaves(), the next node is chosen (node = -1 when none is left), and the ray is finished
     // once its leaves are tested and node < 0; true when it stopped on a bound.
-    template <bool SHARE, class N, class S>
+    template <bool SHARE, bool PAIR = SHARE, class N, class S>
     __device__ __forceinline__ bool visit(const N& nodes, const float4* __restrict__ tv, S& stack, LeafSet& leaves, int& err) {
         if (--budget < 0) { err |= kTravBudget; return true; }
         float4 nf[5]; fetch_node<5>(nodes, node, nf);
@@ -354,8 +354,9 @@ struct CwbvhTrav {
         // factor 2^24 in their exponents (sx24 = 2^(e + 24) / d, exact), so fmaf(q 2^-24, sx24, ox) is bit for bit
         // fmaf(q, 2^e / d, ox) - the slab distances of the reference's decode - at one permute per two planes
         // instead of a permute and a subtraction per plane.
-        // SHARE: the two children of a permute go through one two-wide multiply-add (2% there; the any-hit kernels, which it
-        // costs spills, keep the scalar form)
+        // PAIR: the two children of a permute go through one two-wide multiply-add (with shared triangle tests 1,709 -> 1,669 us on 4.2 M
+        // incoherent rays; in the one-fetch-per-warp loops the camera pass 17.45 -> 16.32 ms and the shadow passes 17.5 -> 16.6 a
+        // 512x512x256 frame). The refilling any-hit loops, which it costs spills, keep the scalar form (435 vs 442 us)
         float2 pbx, pby, pbz, pcx, pcy, pcz;
 #pragma unroll
         for (int s = 0; s < 8; s++) {
@@ -364,7 +365,7 @@ struct CwbvhTrav {
                 pbx = __half22float2(h2_of_bits(__byte_perm(s < 4 ? nx0 : nx1, 0u, sel))); pcx = __half22float2(h2_of_bits(__byte_perm(s < 4 ? px0 : px1, 0u, sel)));
                 pby = __half22float2(h2_of_bits(__byte_perm(s < 4 ? ny0 : ny1, 0u, sel))); pcy = __half22float2(h2_of_bits(__byte_perm(s < 4 ? py0 : py1, 0u, sel)));
                 pbz = __half22float2(h2_of_bits(__byte_perm(s < 4 ? nz0 : nz1, 0u, sel))); pcz = __half22float2(h2_of_bits(__byte_perm(s < 4 ? pz0 : pz1, 0u, sel)));
-                if constexpr (SHARE) {
+                if constexpr (PAIR) {
                     const float2 sx = make_float2(sx24, sx24), sy = make_float2(sy24, sy24), sz = make_float2(sz24, sz24);
                     const float2 o2x = make_float2(ox, ox), o2y = make_float2(oy, oy), o2z = make_float2(oz, oz);
                     pbx = fma2(pbx, sx, o2x); pcx = fma2(pcx, sx, o2x); pby = fma2(pby, sy, o2y); pcy = fma2(pcy, sy, o2y); pbz = fma2(pbz, sz, o2z); pcz = fma2(pcz, sz, o2z);
@@ -372,7 +373,7 @@ struct CwbvhTrav {
             }
             const bool hi = s & 1;
             float xn = hi ? pbx.y : pbx.x, xf = hi ? pcx.y : pcx.x, yn = hi ? pby.y : pby.x, yf = hi ? pcy.y : pcy.x, zn = hi ? pbz.y : pbz.x, zf = hi ? pcz.y : pcz.x;
-            if constexpr (!SHARE) { xn = fmaf(xn, sx24, ox); xf = fmaf(xf, sx24, ox); yn = fmaf(yn, sy24, oy); yf = fmaf(yf, sy24, oy); zn = fmaf(zn, sz24, oz); zf = fmaf(zf, sz24, oz); }
+            if constexpr (!PAIR) { xn = fmaf(xn, sx24, ox); xf = fmaf(xf, sx24, ox); yn = fmaf(yn, sy24, oy); yf = fmaf(yf, sy24, oy); zn = fmaf(zn, sz24, oz); zf = fmaf(zf, sz24, oz); }
             // entry = max(xn, yn, zn, tmin), exit = min(xf, yf, zf, hitT) selected with 3-input integer min/max on the
             // float bits: for values >= +0 the integer order is the float order, entry >= tmin >= +0, and any negative
             // candidate for the exit makes the float comparison below fail whichever negative value is picked - so
@@ -533,7 +534,8 @@ template <bool ANY, int TRI, int FOCT = -1, class N>
 __device__ __forceinline__ bool trav_cwbvh(const N& nodes, const float4* __restrict__ tv, float3 o, float3 d, float tmin,
                                            float& hitT, int& hitTri, float& hu, float& hv, int root, int& err) {
     CwbvhTrav<ANY, TRI, FOCT> r; typename CwbvhTrav<ANY, TRI, FOCT>::Stack stack; r.begin(o, d, tmin, hitT, root);
-    while (!r.step(nodes, tv, stack, err)) {}
+    LeafSet none;
+    while (!r.template visit<false, true>(nodes, tv, stack, none, err)) {}
     hitT = r.hitT; hitTri = r.hitTri; hu = r.hu; hv = r.hv;
     return hitTri >= 0;
 }

@@ -170,7 +170,7 @@ typedef struct cwp_render_options {
     int32_t block;        /* threads per block of the traversal kernels (0 = 128) */
     int32_t device;       /* CUDA device ordinal */
     int32_t profile;      /* 1: CUDA event pair around every kernel launch (also inside the graph), see cwp_renderer_depth_stats */
-    int32_t traversal;    /* 0 auto (refill for CWBVH closest-hit), 1 persistent lanes with dynamic refill everywhere, 2 one 32-ray fetch per warp */
+    int32_t traversal;    /* 0 auto (refill for CWBVH bounces), 1 persistent lanes with dynamic refill everywhere, 2 one 32-ray fetch per warp */
     int32_t sort;         /* continuation rays regrouped before each bounce: 0 off, 1 by direction octant, 2 by octant and a 4x4x4 origin cell */
     int32_t stage_levels; /* CWBVH: levels 0..L of the tree copied into every traversal block's shared memory (L = 1..3, at most
                              512 nodes); -1 none; 0 the library's default */
