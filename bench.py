@@ -865,7 +865,7 @@ def main():
                    clocks=clocks,
                    e2e={"value": e_rays / e_s / 1e9, "unit": "Grays/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": w * h * 16,
                         "note": "scene uploaded once at init; each step renders and reads the w*h float4 accumulation buffer back into pinned host memory"},
-                   gpu_launches=args.steps * (spp // K) * (2 + 2 * depths),
+                   gpu_launches=args.steps * (spp // K) * (1 + 2 * depths),   # pass begin and end, a trace per depth, a shadow pass for all but the last
                    roofline={"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                              "peak_kind": peak_kind, **frame_traffic(args, wl, variant, dom),
                              "algorithmic": f"{STATE_BYTES} B of path state per queued ray read and per continuation/shadow ray written"})
