@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(128, CWPB_TRACE_MINB) k_trace_shade_rf(const _
 // shading decoupled from the refill. Sharing pays while many lanes hold a ray, so the warp refills early; shading then would run
 // with a few lanes each time. Instead a finished ray leaves its path and triangle in a list in shared memory, and the warp
 // shades when the list is full, with all lanes: the ray is read from the queue again, and its distance and barycentrics come from one
-// more test of the triangle (the same arithmetic on the same operands, so the same bits). Camera rays keep k_trace_shade_rf: neighbouring
+// more test of the triangle (the same arithmetic on the same operands, so the same bits). Camera rays test alone: neighbouring
 // rays hit the same leaves in the same step, and sharing their tests measured 25% slower (34.8 vs 27.9 ms).
 #ifndef CWPB_BOUNCE_REFILL
 #define CWPB_BOUNCE_REFILL 6
