@@ -375,16 +375,20 @@ static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_
     b->builder = opt ? opt->builder : 0;
     if (b->builder == 0) { if (int rc = b->blasB.reserve(b->nTris, n)) return rc; }
     // Triangle records, 3 float4 per triangle: (v0, local id), (v1, material), (v2, 0). The meshes go up as they are (half the
-    // bytes of the records) and a kernel gathers them and checks vertex indices and coordinates.
+    // bytes of the records) and a kernel gathers them and checks vertex indices and coordinates. A mesh with more vertices than
+    // corners (a part of a larger vertex array) leaves some unused for certain: its corners are taken out on the host and go up alone,
+    // so that parts sharing one array do not each bring the whole of it.
     {
         std::vector<RawMesh> raw(n);
         long long words = 0;
         for (int m = 0; m < n; m++) {
             const cwp_mesh_view& v = meshes[m];
-            raw[m].vert = words; words += 3 * v.n_verts;
-            raw[m].face = words; words += 3 * v.n_tris;
+            const bool part = v.n_verts > 3 * v.n_tris;
+            raw[m].nVerts = part ? 3 * v.n_tris : v.n_verts;
+            raw[m].vert = words; words += 3 * raw[m].nVerts;
+            raw[m].face = part ? -1 : words; if (!part) words += 3 * v.n_tris;
             raw[m].mat = v.face_mat ? words : -1; if (v.face_mat) words += v.n_tris;
-            raw[m].first = b->meshFirst[m]; raw[m].nVerts = v.n_verts;
+            raw[m].first = b->meshFirst[m];
         }
         unsigned* dWords = nullptr; RawMesh* dRaw = nullptr; unsigned long long* dBad = nullptr;
         auto placeRaw = [&](Carver c) { c.take(dRaw, (size_t)n); c.take(dBad, 1); c.take(dWords, (size_t)words); return c.at; };
@@ -397,8 +401,13 @@ static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_
         if (e == cudaSuccess) e = cudaMemsetAsync(dBad, 0xff, sizeof(unsigned long long), b->st);
         for (int m = 0; m < n && e == cudaSuccess; m++) {
             const cwp_mesh_view& v = meshes[m];
-            e = cudaMemcpyAsync(dWords + raw[m].vert, v.verts, (size_t)v.n_verts * 12, cudaMemcpyHostToDevice, b->st);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(dWords + raw[m].face, v.faces, (size_t)v.n_tris * 12, cudaMemcpyHostToDevice, b->st);
+            std::vector<float> corners;   // (a pageable source: staged before the copy call returns)
+            if (raw[m].face < 0) {
+                corners.assign((size_t)9 * v.n_tris, NAN);   // NaN where the index is out of range: the kernel finds the corner, the check below says why
+                for (int64_t c = 0; c < 3 * v.n_tris; c++) { const int vi = v.faces[c]; if (vi >= 0 && vi < v.n_verts) memcpy(&corners[3 * c], v.verts + 3 * (size_t)vi, 12); }
+            }
+            e = cudaMemcpyAsync(dWords + raw[m].vert, raw[m].face < 0 ? corners.data() : v.verts, (size_t)raw[m].nVerts * 12, cudaMemcpyHostToDevice, b->st);
+            if (e == cudaSuccess && raw[m].face >= 0) e = cudaMemcpyAsync(dWords + raw[m].face, v.faces, (size_t)v.n_tris * 12, cudaMemcpyHostToDevice, b->st);
             if (e == cudaSuccess && v.face_mat) e = cudaMemcpyAsync(dWords + raw[m].mat, v.face_mat, (size_t)v.n_tris * 4, cudaMemcpyHostToDevice, b->st);
         }
         unsigned long long bad = ~0ull;

@@ -25,11 +25,11 @@ __global__ void __launch_bounds__(256) k_gather_triangles(const unsigned* __rest
     const int t = i - m.first;
     float4 v[3];
     for (int k = 0; k < 3; k++) {
-        const int vi = (int)__ldg(words + m.face + 3ll * t + k);
+        const long long vi = m.face < 0 ? 3ll * t + k : (long long)(int)__ldg(words + m.face + 3ll * t + k);
         float3 p = f3(0.f, 0.f, 0.f);
         bool ok = vi >= 0 && vi < m.nVerts;
         if (ok) {
-            const unsigned* q = words + m.vert + 3ll * vi;
+            const unsigned* q = words + m.vert + 3 * vi;
             p = f3(__uint_as_float(__ldg(q)), __uint_as_float(__ldg(q + 1)), __uint_as_float(__ldg(q + 2)));
             ok = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
         }

@@ -33,8 +33,9 @@ void emit_tlas(const SegBuilder& B, int nInst, const int* segFirstDev, int nSeg,
 // World boxes of instances (the 8 corners of their mesh's root box through the object -> world rows).
 void instance_boxes(const cwp_instance* inst, int nInst, const float4* meshBox, float4* lo, float4* hi, cudaStream_t st);
 
-// A batch's meshes as uploaded: mesh m's vertices (3 floats each) from float vert on, its faces (3 ints each) from int face on and its
-// material ids from int mat on (-1: none) in one word array; its triangles are [first, next mesh's first) of the batch.
+// A batch's meshes as uploaded: mesh m's vertices (3 floats each) from float vert on, its faces (3 ints each) from int face on (-1: none,
+// triangle t's corners are vertices 3 t to 3 t + 2) and its material ids from int mat on (-1: none) in one word array; its triangles
+// are [first, next mesh's first) of the batch.
 struct RawMesh { long long vert, face, mat, nVerts; int first; };
 // Triangle records of all meshes (triV: (v0, mesh-local id), (v1, material), (v2, 0)), vertex indices and coordinates checked:
 // *bad (preset to all ones) becomes 4 * triangle + corner of the first offending corner; its record is zero.

@@ -45,3 +45,51 @@ def test_first_bad_corner_is_named(gpu, cwp, mesh, tri, corner, what, builder):
     assert e.value.code == cwp.ERR_INVALID
     text = f"mesh {mesh}: non-finite vertex {f[tri, corner]}" if what == "nan" else f"mesh {mesh} triangle {tri}: vertex index {f[tri, corner]} out of range"
     assert text in str(e.value)
+
+
+def parts(n_verts, counts):
+    """meshes that each use a few vertices of one array of n_verts, from its start to its end, and the same meshes compacted"""
+    big = np.zeros((n_verts, 3), np.float32)   # (pages that nothing touches take no memory)
+    rng = np.random.default_rng(5)
+    shared, alone = [], []
+    for i, n in enumerate(counts):
+        at = (n_verts - 3 * n) * i // max(1, len(counts) - 1)
+        big[at:at + 3 * n] = rng.uniform(-5, 5, (3 * n, 3))
+        f = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
+        mat = np.full(n, i, np.int32)
+        shared.append((big, f + at, mat, None)); alone.append((big[at:at + 3 * n], f, mat, None))
+    return shared, alone
+
+
+def same_layouts(a, b):
+    return all(np.array_equal(x.view(np.uint32), y.view(np.uint32)) for w in (2, 4, 8) for x, y in zip(a.download(w), b.download(w)))
+
+
+@pytest.mark.parametrize("counts", [(1, 2, 3), (255, 1, 257)])
+@pytest.mark.parametrize("builder", [0, 1])
+def test_parts_of_one_vertex_array(gpu, cwp, counts, builder):
+    shared, alone = parts(5000, counts)
+    v, f, m, _ = alone[0]
+    strip_of = (v, np.concatenate([f, f[:1]]), np.concatenate([m, m[:1]]), None)   # and one mesh that goes up as it is
+    assert same_layouts(cwp.Batch(shared + [strip_of], builder=builder), cwp.Batch(alone + [strip_of], builder=builder))
+
+
+def test_parts_of_a_large_vertex_array_fit(gpu, cwp):
+    shared, alone = parts(1 << 27, [4] * 128)   # 1.6 GB of vertices: once per mesh they would be more than the device holds
+    assert same_layouts(cwp.Batch(shared), cwp.Batch(alone))
+
+
+@pytest.mark.parametrize("what", ["index", "negative", "nan"])
+def test_first_bad_corner_of_a_part(gpu, cwp, what):
+    shared, _ = parts(5000, (10, 300))
+    v, f, m, _ = shared[1]
+    f = f.copy()
+    if what == "nan":
+        v[f[7, 1]] = np.nan
+    else:
+        f[7, 1] = len(v) if what == "index" else -1
+    shared[1] = (v, f, m, None)
+    with pytest.raises(cwp.CwpError) as e:
+        cwp.Batch(shared)
+    assert e.value.code == cwp.ERR_INVALID
+    assert (f"mesh 1: non-finite vertex {f[7, 1]}" if what == "nan" else f"mesh 1 triangle 7: vertex index {f[7, 1]} out of range") in str(e.value)
