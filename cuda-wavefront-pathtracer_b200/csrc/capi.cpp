@@ -13,7 +13,9 @@ namespace cwpb {
 static thread_local std::string g_err;
 int set_error(int code, const char* fmt, ...) {
     char buf[1024]; va_list ap; va_start(ap, fmt); vsnprintf(buf, sizeof buf, fmt, ap); va_end(ap);
-    g_err = buf; return code;
+    g_err = buf;
+    if (code == CWP_ERR_NOMEM || code == CWP_ERR_CUDA) cudaGetLastError();   // reported here: the runtime's note of it must not fail the thread's next launch
+    return code;
 }
 void clear_error() { g_err.clear(); }
 }  // namespace cwpb

@@ -1,5 +1,6 @@
 """Shared fixtures: the library under test, the oracle (test infrastructure) and, where built, the reference's own
 code compiled from its sources (oracle/_ref)."""
+import contextlib
 import ctypes as C
 import importlib
 import os
@@ -24,6 +25,18 @@ def has_gpu():
         return torch.cuda.is_available()
     except Exception:
         return False
+
+
+@contextlib.contextmanager
+def only_free(torch, n):
+    """within it, n bytes of device memory are free"""
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - n, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del hold
+        torch.cuda.empty_cache()
 
 
 @pytest.fixture(scope="session")

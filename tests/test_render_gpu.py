@@ -7,7 +7,7 @@ import subprocess
 import numpy as np
 import pytest
 
-from conftest import REF_DIR
+from conftest import REF_DIR, only_free
 
 pytestmark = pytest.mark.gpu
 
@@ -140,3 +140,16 @@ def test_l2_probe(gpu, cwp):
     than an implausible figure."""
     g = cwp.measure_l2_read()
     assert 3000.0 < g < 200000.0
+
+
+def test_a_reported_error_is_over(gpu, cwp):
+    """an allocation that failed and was reported does not fail the next frame (or another library's next launch)"""
+    mesh, bvh = cwp.scene("boxes12k", variant=8, bins=32)
+    r = cwp.Renderer()
+    with only_free(gpu, 256 << 20):
+        with pytest.raises(cwp.CwpError) as e:
+            r.init(cwp.frame_params(mesh, 2048, 1024), bvh, variant=8, batch=4)   # 8.4 M paths: 1 GB
+        assert e.value.code == cwp.ERR_NOMEM
+        r.init(cwp.frame_params(mesh, 64, 48), bvh, variant=8, batch=4)
+        assert r.render(4).rays > 0
+    assert gpu.ones(3, device="cuda").sum().item() == 3.0
