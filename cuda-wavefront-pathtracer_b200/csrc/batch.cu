@@ -537,6 +537,7 @@ extern "C" int cwp_batch_set_scenes(cwp_batch* b, const cwp_instance* inst, int6
     const int nSeg = (int)seg.size() - 1;
     CWPB_CHECK(nSeg <= (1 << kSegBits), CWP_ERR_INVALID, "%d non-empty scenes (limit %d)", nSeg, 1 << kSegBits);
     CWPB_CUDA(cudaSetDevice(b->device));
+    b->nScenes = 0;   // not traceable until the new TLAS passes its check, whichever step fails before that
     if (int rc = ensure_scene_arrays(b, n, nScenes)) return rc;
     CWPB_CUDA(cudaEventRecord(b->e0, b->st));
     if (n > 0) CWPB_CUDA(cudaMemcpyAsync(b->inst, inst, (size_t)n * sizeof(cwp_instance), cudaMemcpyHostToDevice, b->st));
@@ -549,7 +550,7 @@ extern "C" int cwp_batch_set_scenes(cwp_batch* b, const cwp_instance* inst, int6
     }
     CWPB_CUDA(cudaEventRecord(b->e1, b->st));
     CWPB_CUDA(cudaGetLastError());
-    b->nScenes = 0;   // not traceable until the new TLAS passes its check (which waits for the stream)
+    // the check waits for the stream
     if (int rc = check_tlas(b->tlas, (int)n, b->segFirstTlas, nSeg, b->err, b->st, nullptr, b->tlas4)) return rc;
     float ms = 0; CWPB_CUDA(cudaEventElapsedTime(&ms, b->e0, b->e1)); b->tlasMs = ms;
     b->nScenes = nScenes; b->nInst = n; b->sceneFirst.assign(first, first + nScenes + 1); b->fixedCap = 0;

@@ -5,6 +5,8 @@ agreement across widths and tunings, per-frame TLAS rebuilds, and the autotuner.
 import numpy as np
 import pytest
 
+from conftest import only_free
+
 pytestmark = pytest.mark.gpu
 
 
@@ -266,3 +268,34 @@ def test_incremental_scene_updates_match_packed(gpu, cwp):
         b.update_scenes([1, 1], None, [0, 0])   # listed twice
     with pytest.raises(Exception):
         arr, cnt = part([1]); b.update_scenes([4], arr, cnt)   # out of range
+
+
+def test_scenes_without_memory_are_not_traced(gpu, cwp):
+    """set_scenes that finds no memory for its arrays has freed the old ones: a trace then is refused, and works again after the
+    next set_scenes"""
+    v = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0]], np.float32)
+    b = cwp.Batch([(v, np.array([[0, 1, 2]], np.int32), None, None)])
+    one = np.eye(3, 4, dtype=np.float32).reshape(1, 12)
+    few = cwp.instances(one, [0])
+    many = (cwp.Instance * (1 << 21))()
+    np.frombuffer(many, np.uint8).reshape(-1, 112)[:] = np.frombuffer(few, np.uint8)
+    ray = [gpu.tensor([x], dtype=gpu.float32, device="cuda") for x in ([0.2, 0.2, 1.0, 0.0], [0.0, 0.0, -1.0, 10.0])]
+    sc, who = gpu.zeros(1, dtype=gpu.int32, device="cuda"), gpu.full((1,), -7, dtype=gpu.int32, device="cuda")
+    hits = gpu.zeros(1, 4, device="cuda")
+
+    def trace():
+        b.trace(ray[0].data_ptr(), ray[1].data_ptr(), sc.data_ptr(), hits.data_ptr(), who.data_ptr(), 1)
+        gpu.cuda.synchronize(); b.status()
+        return hits.cpu().numpy()[0, 0], int(who.cpu()[0])
+
+    b.set_scenes(few, [0, 1])
+    assert trace() == (1.0, 0)
+    with only_free(gpu, 128 << 20):
+        with pytest.raises(cwp.CwpError) as e:
+            b.set_scenes(many, [0, len(many)])     # 235 MB of instances alone
+        assert e.value.code == cwp.ERR_NOMEM
+        with pytest.raises(cwp.CwpError) as e:
+            trace()
+        assert e.value.code == cwp.ERR_STATE
+    b.set_scenes(few, [0, 1])
+    assert trace() == (1.0, 0)
