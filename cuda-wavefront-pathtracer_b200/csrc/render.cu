@@ -680,8 +680,8 @@ int ensure_events(cwp_renderer* r, int passes) {
 
 // All passes of a frame with device-side queue lengths and persistent grids (the captured sequence). Every launch of a small
 // pass ends in a tail: its queue is empty and a few long rays hold the GPU. With r->beside the shadow pass of a depth is a
-// branch of the graph beside the next depth's trace+shade, on a stream of lower priority, and fills that tail; the branches
-// join at the end of the pass. It needs a shadow queue per depth, so it is taken up to kBesideEntries queue entries (672 MB);
+// branch of the graph beside the next depth's trace+shade and fills that tail; the branches join at the end of the pass (a
+// higher priority for the trace gave nothing: 8,905 and 8,901 us for four 720p samples, 1,123 and 1,124 for 256x256x16). It needs a shadow queue per depth, so it is taken up to kBesideEntries queue entries (672 MB);
 // larger passes lose under 1% to tails.
 static constexpr long long kBesideEntries = 1ll << 24;
 int enqueue_passes(cwp_renderer* r, int spp) {
@@ -754,12 +754,10 @@ extern "C" int cwp_renderer_init(cwp_renderer* r, const cwp_params* p, const cwp
     r->P = *p; r->O = *o;
     r->N = p->cam.w * p->cam.h; r->K = o->batch; r->nk = nk; r->depths = o->bounces + 2;
     if (!r->shadowed) {
-        int least = 0, greatest = 0;
-        CWPB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        if (!r->st) CWPB_CUDA(cudaStreamCreateWithPriority(&r->st, cudaStreamNonBlocking, greatest < least ? least - 1 : least));
+        if (!r->st) CWPB_CUDA(cudaStreamCreateWithFlags(&r->st, cudaStreamNonBlocking));
         if (!r->f0) CWPB_CUDA(cudaEventCreate(&r->f0));
         if (!r->f1) CWPB_CUDA(cudaEventCreate(&r->f1));
-        if (!r->st2) CWPB_CUDA(cudaStreamCreateWithPriority(&r->st2, cudaStreamNonBlocking, least));
+        if (!r->st2) CWPB_CUDA(cudaStreamCreateWithFlags(&r->st2, cudaStreamNonBlocking));
         if (!r->traced) CWPB_CUDA(cudaEventCreateWithFlags(&r->traced, cudaEventDisableTiming));
         CWPB_CUDA(cudaEventCreateWithFlags(&r->shadowed, cudaEventDisableTiming));
     }
