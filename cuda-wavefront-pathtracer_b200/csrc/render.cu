@@ -606,14 +606,14 @@ template <int V, int TRI, bool STAGE = false> int occupancy_of(int& bt0, int& bt
 }
 
 // ev: 4 events (trace start/end, shadow start/end) or nullptr
-template <int V, int TRI, bool STAGE = false> void launch_depth(cwp_renderer* r, KArgs a, int gt0, int gt, int gs, cudaEvent_t* ev, bool beside) {
+template <int V, int TRI, bool STAGE = false> int launch_depth(cwp_renderer* r, KArgs a, int gt0, int gt, int gs, cudaEvent_t* ev, bool beside) {
     const cudaStream_t ss = beside ? r->st2 : r->st;   // the shadow pass's stream
     const bool shadows = a.depth <= r->P.max_b;        // a path's last hit casts none
     // external records: inside a stream capture they become event-record nodes of the graph
     bool rf = false, rfShadow = false;
     const size_t sm = STAGE ? (size_t)80 * a.staged : 0;
     if constexpr (V != 4) { rf = r->refill; rfShadow = r->refillShadow; }
-    if (ev) cudaEventRecordWithFlags(ev[0], r->st, cudaEventRecordExternal);
+    if (ev) CWPB_CUDA(cudaEventRecordWithFlags(ev[0], r->st, cudaEventRecordExternal));
     const bool escape = a.depth > 0 && a.depth > r->P.max_b;
     if (escape) k_escape<V, TRI, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
     if constexpr (V != 4) {
@@ -636,8 +636,8 @@ template <int V, int TRI, bool STAGE = false> void launch_depth(cwp_renderer* r,
         k_sort_scan<<<1, kSortBins, 0, r->st>>>(sa);
         k_sort_scatter<<<r->nSM * 8, 256, 0, r->st>>>(sa);
     }
-    if (ev) { cudaEventRecordWithFlags(ev[1], r->st, cudaEventRecordExternal); cudaEventRecordWithFlags(ev[2], r->st, cudaEventRecordExternal); }
-    if (beside) { cudaEventRecord(r->traced, r->st); cudaStreamWaitEvent(r->st2, r->traced, 0); }
+    if (ev) { CWPB_CUDA(cudaEventRecordWithFlags(ev[1], r->st, cudaEventRecordExternal)); CWPB_CUDA(cudaEventRecordWithFlags(ev[2], r->st, cudaEventRecordExternal)); }
+    if (beside) { CWPB_CUDA(cudaEventRecord(r->traced, r->st)); CWPB_CUDA(cudaStreamWaitEvent(r->st2, r->traced, 0)); }   // without the wait the shadow pass would read a queue still being filled
     if constexpr (V != 4) { if (rfShadow && shadows) k_shadow_rf<V, TRI, STAGE><<<gs, 128, sm, ss>>>(a); }
     if (!rfShadow && shadows) {
         int foct = -1;
@@ -649,7 +649,8 @@ template <int V, int TRI, bool STAGE = false> void launch_depth(cwp_renderer* r,
             default: k_shadow<V, TRI, STAGE><<<gs, 128, sm, ss>>>(a);
         }
     }
-    if (ev) cudaEventRecordWithFlags(ev[3], r->st, cudaEventRecordExternal);
+    if (ev) CWPB_CUDA(cudaEventRecordWithFlags(ev[3], r->st, cudaEventRecordExternal));
+    return CWP_OK;
 }
 
 KArgs base_args(cwp_renderer* r) {
@@ -659,15 +660,15 @@ KArgs base_args(cwp_renderer* r) {
     return a;
 }
 
-void dispatch_depth(cwp_renderer* r, KArgs a, int gt0, int gt, int gs, int pass, bool beside = false) {
+int dispatch_depth(cwp_renderer* r, KArgs a, int gt0, int gt, int gs, int pass, bool beside = false) {
     if (beside) { const size_t at = (size_t)a.depth * r->nk; a.q.h0 += at; a.q.h1 += at; a.q.h2 += at; }   // the depth's own shadow queue
     const int V = r->scene.variant, T = r->scene.tri;
     if (r->O.sort && a.depth > 0) { const int rd = a.depth & 1; a.q.s0[rd] = r->t0; a.q.s1[rd] = r->t1; a.q.s2[rd] = r->t2; }
     cudaEvent_t* ev = r->O.profile ? &r->ev[((size_t)pass * r->depths + a.depth) * 4] : nullptr;
-    if (V == 2) { if (T) launch_depth<2, 1>(r, a, gt0, gt, gs, ev, beside); else launch_depth<2, 0>(r, a, gt0, gt, gs, ev, beside); }
-    else if (V == 4) { if (T) launch_depth<4, 1>(r, a, gt0, gt, gs, ev, beside); else launch_depth<4, 0>(r, a, gt0, gt, gs, ev, beside); }
-    else if (r->staged) { if (T) launch_depth<8, 1, true>(r, a, gt0, gt, gs, ev, beside); else launch_depth<8, 0, true>(r, a, gt0, gt, gs, ev, beside); }
-    else { if (T) launch_depth<8, 1>(r, a, gt0, gt, gs, ev, beside); else launch_depth<8, 0>(r, a, gt0, gt, gs, ev, beside); }
+    if (V == 2) return T ? launch_depth<2, 1>(r, a, gt0, gt, gs, ev, beside) : launch_depth<2, 0>(r, a, gt0, gt, gs, ev, beside);
+    if (V == 4) return T ? launch_depth<4, 1>(r, a, gt0, gt, gs, ev, beside) : launch_depth<4, 0>(r, a, gt0, gt, gs, ev, beside);
+    if (r->staged) return T ? launch_depth<8, 1, true>(r, a, gt0, gt, gs, ev, beside) : launch_depth<8, 0, true>(r, a, gt0, gt, gs, ev, beside);
+    return T ? launch_depth<8, 1>(r, a, gt0, gt, gs, ev, beside) : launch_depth<8, 0>(r, a, gt0, gt, gs, ev, beside);
 }
 
 // profiling events for `passes` passes (created on first need, kept)
@@ -692,7 +693,7 @@ int enqueue_passes(cwp_renderer* r, int spp) {
         KArgs a = base_args(r); a.sBase = s; a.sDev = r->cnt + nInts;
         for (int d = 0; d < r->depths; d++) {
             a.depth = d;
-            dispatch_depth(r, a, r->gridTrace0, r->gridTrace, r->gridShadow, pass, beside && d < r->depths - 1);
+            if (int rc = dispatch_depth(r, a, r->gridTrace0, r->gridTrace, r->gridShadow, pass, beside && d < r->depths - 1)) return rc;
         }
         if (beside) { CWPB_CUDA(cudaEventRecord(r->shadowed, r->st2)); CWPB_CUDA(cudaStreamWaitEvent(r->st, r->shadowed, 0)); }
         k_pass_end<<<1, 32, 0, r->st>>>(r->cnt, r->depths, r->tot);
@@ -895,7 +896,7 @@ extern "C" int cwp_renderer_render(cwp_renderer* r, int32_t spp, cwp_frame_stats
                 a.depth = d;
                 const int need = (n + 127) / 128;
                 const int gt = need < r->gridTrace ? need : r->gridTrace, gt0 = need < r->gridTrace0 ? need : r->gridTrace0;
-                dispatch_depth(r, a, gt0, gt, r->gridShadow, pass);
+                if (int rc = dispatch_depth(r, a, gt0, gt, r->gridShadow, pass)) return rc;
                 CWPB_CUDA(cudaMemcpyAsync(r->hcnt, r->cnt, (size_t)nInts * sizeof(int), cudaMemcpyDeviceToHost, r->st));
                 CWPB_CUDA(cudaStreamSynchronize(r->st));
                 n = r->hcnt[4 * (d + 1)];
