@@ -682,12 +682,14 @@ int ensure_events(cwp_renderer* r, int passes) {
 // All passes of a frame with device-side queue lengths and persistent grids (the captured sequence). Every launch of a small
 // pass ends in a tail: its queue is empty and a few long rays hold the GPU. With r->beside the shadow pass of a depth is a
 // branch of the graph beside the next depth's trace+shade and fills that tail; the branches join at the end of the pass (a
-// higher priority for the trace gave nothing: 8,905 and 8,901 us for four 720p samples, 1,123 and 1,124 for 256x256x16). It needs a shadow queue per depth, so it is taken up to kBesideEntries queue entries (672 MB);
-// larger passes lose under 1% to tails.
+// higher priority for the trace gave nothing: 8,905 and 8,901 us for four 720p samples, 1,123 and 1,124 for 256x256x16). It needs a shadow queue per depth, so it is taken up to kBesideEntries queue entries (672 MB;
+// larger passes lose under 1% to tails), and only where the queues are at most 1 / kBesideShare of the free memory: a form that
+// is merely faster must not take what the program allocates next.
 static constexpr long long kBesideEntries = 1ll << 24;
+static constexpr size_t kBesideShare = 16;
 int enqueue_passes(cwp_renderer* r, int spp) {
     const int nInts = 4 * (r->depths + 1);
-    const bool beside = r->beside && !r->O.profile;   // (per-kernel times need the kernels one after another)
+    const bool beside = r->beside;
     for (int s = 0, pass = 0; s < spp; s += r->K, pass++) {
         k_pass_begin<<<1, 128, 0, r->st>>>(r->cnt, nInts, (int)r->nk, r->sortBins, r->sortBins ? 2 * kSortBins * r->depths : 0);
         KArgs a = base_args(r); a.sBase = s; a.sDev = r->cnt + nInts;
@@ -791,14 +793,18 @@ extern "C" int cwp_renderer_init(cwp_renderer* r, const cwp_params* p, const cwp
     if (!rc) rc = alloc((void**)&r->tot, (2 * (size_t)r->depths + 1) * sizeof(unsigned long long));   // and the status word
     if (rc) return rc;
     r->err = reinterpret_cast<int*>(r->tot + 2 * r->depths);
-    // shadow queues: one per depth where shadow passes run beside the next bounce and the memory is there, else one
+    // shadow queues: one per depth where shadow passes run beside the next bounce (not with per-kernel times, which need the kernels
+    // one after another) and there is memory to spare, else one
     r->beside = false;
-    if (o->graph && o->bounces >= 1 && nk * (o->bounces + 1) <= kBesideEntries) {
+    if (o->graph && !o->profile && o->bounces >= 1 && nk * (o->bounces + 1) <= kBesideEntries) {
         const size_t NE = NK * (o->bounces + 1); void* h = nullptr;
-        if (cudaMalloc(&h, NE * 40) == cudaSuccess) {
-            r->allocs.push_back(h); r->beside = true;
-            r->q.h0 = (float4*)h; r->q.h1 = r->q.h0 + NE; r->q.h2 = (float2*)(r->q.h1 + NE);
-        } else cudaGetLastError();
+        size_t spare = 0; CWPB_CUDA(cudaMemGetInfo(&spare, &total));
+        if (NE * 40 <= spare / kBesideShare) {
+            if (cudaMalloc(&h, NE * 40) == cudaSuccess) {
+                r->allocs.push_back(h); r->beside = true;
+                r->q.h0 = (float4*)h; r->q.h1 = r->q.h0 + NE; r->q.h2 = (float2*)(r->q.h1 + NE);
+            } else cudaGetLastError();
+        }
     }
     if (!r->beside) {
         rc = alloc((void**)&r->q.h0, NK * 16);

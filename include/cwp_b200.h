@@ -143,6 +143,9 @@ int cwp_trace_fp64(cwp_accel* a, int32_t any_hit, const float* d_o, const float*
  * render (wavefront.cu:684-741 legacy loop, 644-680 graph frame), readAccum / accumDevice (renderer.h:58-59),
  * setParams / setMaterials (wavefront.cu:744-752), introspection (renderer.h:69). Params mirrors render/params.h:8-16,
  * RenderOptions renderer.h:11-28, FrameStats renderer.h:45. The accumulation buffer holds w*h float4 radiance sums.
+ * Device memory beyond the scene: 120 B per path in flight (w*h*batch; 160 with sort); graph frames without profile
+ * whose paths times bounces + 1 are at most 2^24 take 40 B per path for each bounce more, where that is at most a
+ * sixteenth of the free memory.
  * ------------------------------------------------------------------------------------------------------------------ */
 typedef struct cwp_camera {
     float pos[3], ax[3], ay[3], az[3];   /* camera looks down -az, +ay up (scene/camera.h:7) */

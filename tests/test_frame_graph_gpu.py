@@ -3,6 +3,8 @@ range, at image sizes and depths where a branch or a queue can be empty."""
 import numpy as np
 import pytest
 
+from conftest import only_free
+
 pytestmark = pytest.mark.gpu
 
 
@@ -22,3 +24,20 @@ def test_graph_frame_equals_host_loop(gpu, cwp, variant, w, h, batch, bounces):
         # rounds by at most 2^-24 of the sum
         n = 6 * batch * (bounces + 2) * 2
         assert np.all(np.abs(x - y) <= n * 2.0 ** -24 * np.maximum(np.abs(y), 1e-30) * 2)
+
+
+def test_scarce_memory_keeps_one_shadow_queue(gpu, cwp):
+    """a shadow queue per depth is taken from plenty only: with little memory free the frame keeps one and is the same"""
+    mesh, bvh = cwp.scene(64, variant=8, bins=16)
+    w, h, bounces = 1024, 512, 4                       # 0.5 M paths: 21 MB a queue, 105 MB for all depths
+    p = cwp.frame_params(mesh, w, h, bounces=bounces)
+    roomy, scarce = cwp.Renderer(), cwp.Renderer()
+    roomy.init(p, bvh, variant=8, batch=1, bounces=bounces)
+    with only_free(gpu, 1 << 30):
+        scarce.init(p, bvh, variant=8, batch=1, bounces=bounces)
+    assert roomy.info().vram_mb - scarce.info().vram_mb >= 0.9 * bounces * 40 * w * h / 2 ** 20
+    a, b = roomy.render(4), scarce.render(4)
+    assert (a.rays, a.shadow_rays) == (b.rays, b.shadow_rays)
+    x, y = roomy.read_accum(), scarce.read_accum()
+    n = 4 * (bounces + 2) * 2   # the same float contributions in another order, as above
+    assert np.all(np.abs(x - y) <= n * 2.0 ** -24 * np.maximum(np.abs(y), 1e-30) * 2)
