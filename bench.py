@@ -751,7 +751,7 @@ def main():
     ap.add_argument("--tuning", default="", help="batched64 / serving: fixed launch shape block,width,fetch,smem (batched64: instead of the autotuner)")
     ap.add_argument("--builder", type=int, default=0, help="batched64: 0 every BLAS on the GPU (H-PLOC, one launch), 1 on the host cores (binned SAH)")
     ap.add_argument("--precision", action="store_true", help="ray-batch workloads: use the precision form")
-    ap.add_argument("--traversal", type=int, default=0, help="0 auto (persistent refill for BVH2/CWBVH), 1 refill, 2 one 32-ray fetch per warp")
+    ap.add_argument("--traversal", type=int, default=0, help="0 auto (refill for CWBVH bounces and the rays beyond the bounce limit), 1 refill, 2 one fetch of up to 32 rays per warp")
     ap.add_argument("--spatial", type=float, default=1e-3, help="host BVH: spatial-split overlap threshold (1e-3 = SBVH, the default; 0 = the reference binned SAH only)")
     ap.add_argument("--paths", type=int, default=0, help="serving: paths in flight over all requests (default: the workload's; profiling cases)")
     ap.add_argument("--max-requests", type=int, default=0, help="serving: requests admitted at once by the continuous form (default: the workload's)")

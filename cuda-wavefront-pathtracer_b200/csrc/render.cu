@@ -6,12 +6,15 @@
 //   both: closest-hit traversal, then shading: miss -> sky; hit at depth <= bounces -> sun next-event estimation into
 //   the shadow queue and a cosine continuation into the next depth's queue, both appended by one atomic per warp
 //   (ballot + popc) so that every warp writes a contiguous run;
+//   k_bounce<depth > 0> over a CWBVH: the same with refilled lanes and triangle tests shared over the warp;
+//   k_escape<depth > bounces>: any-hit traversal, the sky where nothing is hit (a hit there ends the path with nothing);
 //   k_shadow: any-hit traversal of the shadow queue, unoccluded contributions added with one float4 atomic each.
 // The semantics are those of the reference's legacy path (render/wavefront.cu:42-58 raygen, 94-136 shadeOne,
 // 684-741 frame loop): same sample streams (pixel, sample, depth, dimension), same per-vertex decisions, so frames
 // agree sample by sample with the reference's up to rounding.
-// All traversal kernels are persistent (grid = resident blocks) with per-warp dynamic fetching of 32 paths, and read
-// their queue lengths from device memory, so a whole frame is captured once as a CUDA graph and replayed.
+// All traversal kernels are persistent (grid = resident blocks), each warp fetching up to 32 paths at a time or refilling
+// its idle lanes, and read their queue lengths from device memory, so a whole frame is captured once as a CUDA graph and
+// replayed.
 #include "scene_dev.h"
 #include "trav.cuh"
 #include <algorithm>
@@ -614,7 +617,7 @@ template <int V, int TRI, bool STAGE = false> int launch_depth(cwp_renderer* r, 
     const size_t sm = STAGE ? (size_t)80 * a.staged : 0;
     if constexpr (V != 4) { rf = r->refill; rfShadow = r->refillShadow; }
     if (ev) CWPB_CUDA(cudaEventRecordWithFlags(ev[0], r->st, cudaEventRecordExternal));
-    const bool escape = a.depth > 0 && a.depth > r->P.max_b;
+    const bool escape = a.depth > 0 && a.depth > r->P.max_b && r->O.traversal != 2;   // (2 asks for one fetch per warp at every depth)
     if (escape) k_escape<V, TRI, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
     if constexpr (V != 4) {
         if (rf && !escape) {
@@ -1062,7 +1065,7 @@ extern "C" int cwp_render_noalloc(const cwp_params* p, const cwp_device_scene* s
     CWPB_CHECK(o->bounces >= 0 && o->bounces <= kNoAllocMaxBounces, CWP_ERR_INVALID, "bounces %d outside [0, %d] of the no-allocation path", o->bounces, kNoAllocMaxBounces);
     CWPB_CHECK(p->max_b <= o->bounces, CWP_ERR_INVALID, "params max_b %d exceeds bounces %d", p->max_b, o->bounces);
     CWPB_CHECK(spp > 0 && spp % o->batch == 0 && s_base >= 0, CWP_ERR_INVALID, "spp %d must be a positive multiple of batch %d", spp, o->batch);
-    CWPB_CHECK(o->traversal == 0 || o->traversal == 2, CWP_ERR_INVALID, "traversal %d: the no-allocation path runs one 32-ray fetch per warp (0 or 2)", o->traversal);
+    CWPB_CHECK(o->traversal == 0 || o->traversal == 2, CWP_ERR_INVALID, "traversal %d: the no-allocation path has no refill traversal of camera rays and bounces (0 or 2)", o->traversal);
     CWPB_CHECK(o->sort == 0, CWP_ERR_INVALID, "sort %d: the no-allocation path has no regrouping buffers (sort must be 0)", o->sort);
     int dev = 0; CWPB_CUDA(cudaGetDevice(&dev));
     CWPB_CHECK(o->device == dev, CWP_ERR_INVALID, "options.device %d is not the current device %d (make it current before the call)", o->device, dev);
@@ -1096,7 +1099,7 @@ extern "C" int cwp_render_noalloc(const cwp_params* p, const cwp_device_scene* s
         for (int d = 0; d < depths; d++) {
             a.depth = d;
 #define CWPB_NA(VV, TT) do { if (d == 0) k_trace_shade<VV, TT, true><<<na.gridTrace0, 128, 0, st>>>(a, *p); \
-                             else if (d > p->max_b) k_escape<VV, TT><<<na.gridTrace, 128, 0, st>>>(a, *p); \
+                             else if (d > p->max_b && o->traversal != 2) k_escape<VV, TT><<<na.gridTrace, 128, 0, st>>>(a, *p); \
                              else k_trace_shade<VV, TT, false><<<na.gridTrace, 128, 0, st>>>(a, *p); \
                              if (d + 1 < depths) k_shadow<VV, TT><<<na.gridShadow, 128, 0, st>>>(a); } while (0)
             if (o->variant == 2) { if (o->tri) CWPB_NA(2, 1); else CWPB_NA(2, 0); }

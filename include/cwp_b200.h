@@ -173,7 +173,9 @@ typedef struct cwp_render_options {
     int32_t block;        /* threads per block of the traversal kernels (0 = 128) */
     int32_t device;       /* CUDA device ordinal */
     int32_t profile;      /* 1: CUDA event pair around every kernel launch (also inside the graph), see cwp_renderer_depth_stats */
-    int32_t traversal;    /* 0 auto (refill for CWBVH bounces), 1 persistent lanes with dynamic refill everywhere, 2 one 32-ray fetch per warp */
+    int32_t traversal;    /* 0 auto (refill for CWBVH bounces and, in every layout, for the any-hit traversal of the rays beyond the
+                             bounce limit), 1 persistent lanes with dynamic refill everywhere, 2 everywhere one fetch of up to 32
+                             rays per warp at a time, traversed to the end */
     int32_t sort;         /* continuation rays regrouped before each bounce: 0 off, 1 by direction octant, 2 by octant and a 4x4x4 origin cell */
     int32_t stage_levels; /* CWBVH: levels 0..L of the tree copied into every traversal block's shared memory (L = 1..3, at most
                              512 nodes); -1 none; 0 the library's default */
@@ -212,9 +214,10 @@ void cwp_renderer_destroy(cwp_renderer* r);
  * stream-ordered on `stream`; when h_rays is not NULL the call waits for the frame and stores the closest and shadow
  * ray totals there (and reports traversal errors). The call runs on the current device: options.device must name
  * it, and every scene pointer and d_accum must be device (or managed) memory of that device, else CWP_ERR_INVALID.
- * Of the options, variant, tri, batch, bounces and device are used; the traversal is always one 32-ray fetch per
- * warp (traversal must be 0 or 2), there is no regrouping (sort must be 0), and graph, block and profile are
- * ignored: the passes are plain stream launches.
+ * Of the options, variant, tri, batch, bounces and device are used; camera rays and bounces run one 32-ray fetch per
+ * warp, the rays beyond the bounce limit any-hit traversal with refill (traversal 0) or one fetch per warp too
+ * (traversal 2; 1 is refused); there is no regrouping (sort must be 0), and graph, block and profile are ignored: the
+ * passes are plain stream launches.
  * ------------------------------------------------------------------------------------------------------------------ */
 typedef struct cwp_device_scene {
     const float* nodes; const float* tris; const float* woop; const float* nrm;   /* device pointers; woop / nrm may be NULL */
