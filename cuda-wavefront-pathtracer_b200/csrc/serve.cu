@@ -485,8 +485,9 @@ struct cwp_server {
     float* ftab = nullptr;   // Blackman-Harris pixel-filter inverse CDF (CWP_FILTER_TABLE + 1 floats)
     RayQueue q[2]{}; RayQueue qs{}; int* slotBins = nullptr; float4* hits = nullptr; int* hinst = nullptr; int4* dChunks = nullptr;
     // Shadow rays beside the next step: a step's any-hit launch and accumulation run on st2 while the host takes the step's counts
-    // and the next step's closest hits are traced, so queue, results and counts alternate between two sets (one without memory for two)
-    ShadowQueue sq[2]{}; int* occ[2] = { nullptr, nullptr }; int* cnt[2] = { nullptr, nullptr }; bool beside = false; int par = 0;
+    // and the next step's closest hits are traced, so queue, results and counts alternate between two sets (one without memory for two).
+    // The second is only lent: what a request or a table needs comes first (give_back)
+    ShadowQueue sq[2]{}; int* occ[2] = { nullptr, nullptr }; int* cnt[2] = { nullptr, nullptr }; bool beside = false; int par = 0; void* second = nullptr;
     cudaStream_t st2 = nullptr; cudaEvent_t shaded = nullptr, evS[2][3] = {};   // per set: shadow start, accumulation start, end
     bool shadowTimed[2] = { true, true };   // the set's last times are in info (false: to be taken once its end has passed)
     int* hcnt = nullptr;   // pinned: [0..1] counts, then slot counters
@@ -542,6 +543,38 @@ static int make_textures(const cwp_texture* tex, int n, std::vector<cudaArray_t>
 
 static double now_ms(const cwp_server* s) { return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - s->t0).count(); }
 
+// adds a set's shadow times to the statistics once (waits for its end)
+static int take_shadow_times(cwp_server* s, int p) {
+    if (s->shadowTimed[p]) return CWP_OK;
+    s->shadowTimed[p] = true;
+    float d = 0, e = 0;
+    CWPB_CUDA(cudaEventSynchronize(s->evS[p][2]));
+    CWPB_CUDA(cudaEventElapsedTime(&d, s->evS[p][0], s->evS[p][2])); CWPB_CUDA(cudaEventElapsedTime(&e, s->evS[p][1], s->evS[p][2]));
+    s->info.shadow_ms += d; s->info.accum_ms += e;
+    return CWP_OK;
+}
+
+// Frees the second shadow set: from the next step on the shadow pass follows the shading on one stream. Called between steps,
+// when something else needs the memory; true when there was a set to free.
+static int give_back(cwp_server* s, bool& freed) {
+    freed = false;
+    if (!s->beside) return CWP_OK;
+    CWPB_CUDA(cudaStreamSynchronize(s->st)); CWPB_CUDA(cudaStreamSynchronize(s->st2));
+    for (int p = 0; p < 2; p++) if (int rc = take_shadow_times(s, p)) return rc;
+    s->beside = false; s->par = 0;
+    CWPB_CUDA(cudaFree(s->second)); s->second = nullptr;
+    s->freeAt = -1e30;   // the last free-memory query is out of date
+    freed = true;
+    return CWP_OK;
+}
+// f() once more without the second shadow set when there was no memory for it
+template <class F> static int with_room(cwp_server* s, F f) {
+    int rc = f();
+    bool freed = false;
+    if (rc == CWP_ERR_NOMEM && s) { if (int r2 = give_back(s, freed)) return r2; if (freed) rc = f(); }
+    return rc;
+}
+
 extern "C" double cwp_server_clock_ms(const cwp_server* s) { return s ? now_ms(s) : 0.0; }
 
 extern "C" void cwp_server_destroy(cwp_server* s) {
@@ -560,6 +593,7 @@ extern "C" void cwp_server_destroy(cwp_server* s) {
     free_textures(s->texArrays, s->texObjs);
     cudaFree(s->dTexObj); cudaFree(s->dMtex); cudaFree(s->dUvs); cudaFree(s->dTans);
     for (void* p : s->allocs) cudaFree(p);
+    cudaFree(s->second);
     if (s->hcnt) cudaFreeHost(s->hcnt);
     if (s->hSlots) cudaFreeHost(s->hSlots);
     if (s->hChunks) cudaFreeHost(s->hChunks);
@@ -633,14 +667,13 @@ static int server_create(cwp_batch* b, const cwp_material* mats, int n, const in
         uint64_t keep = UINT64_MAX;   // never hand freed images back to the driver between steps
         CWPB_CUDA(cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     }
-    // the second shadow set, where it leaves the reserve untouched
-    {
+    // the second shadow set, where it leaves the reserve untouched and steps overlap (otherwise each waits for its own shadow pass)
+    if (s->overlap) {
         size_t freeB = 0, totalB = 0;
         CWPB_CUDA(cudaMemGetInfo(&freeB, &totalB));
-        void* second = nullptr;
         if ((int64_t)freeB - (int64_t)shadowBytes > s->O.hbm_reserve) {
-            if (cudaMalloc(&second, shadowBytes) == cudaSuccess) { s->allocs.push_back(second); placeShadow(1, Carver(second)); s->beside = true; }
-            else cudaGetLastError();
+            if (cudaMalloc(&s->second, shadowBytes) == cudaSuccess) { placeShadow(1, Carver(s->second)); s->beside = true; }
+            else { cudaGetLastError(); s->second = nullptr; }
         }
     }
     CWPB_CUDA(cudaMemcpy(s->mats, mats, (size_t)n * sizeof(cwp_material), cudaMemcpyHostToDevice));
@@ -666,7 +699,7 @@ extern "C" int cwp_server_create(cwp_batch* b, const cwp_material* mats, int32_t
     return CWP_OK;
 }
 
-extern "C" int cwp_server_set_scenes(cwp_server* s, const cwp_instance_desc* desc, int64_t n, const int32_t* first, int32_t nScenes) {
+static int set_scenes(cwp_server* s, const cwp_instance_desc* desc, int64_t n, const int32_t* first, int32_t nScenes) {
     CWPB_CHECK(s && first && nScenes >= 1 && (n == 0 || desc), CWP_ERR_INVALID, "NULL argument");
     CWPB_CHECK(first[0] == 0 && first[nScenes] == n, CWP_ERR_INVALID, "scene offsets do not cover the %lld descriptors", (long long)n);
     for (int k = 0; k < nScenes; k++) CWPB_CHECK(first[k + 1] >= first[k], CWP_ERR_INVALID, "scene offsets decrease at %d", k);
@@ -680,6 +713,9 @@ extern "C" int cwp_server_set_scenes(cwp_server* s, const cwp_instance_desc* des
     s->desc.assign(desc, desc + n); s->sceneFirst.assign(first, first + nScenes + 1);
     s->xf.clear(); s->xfFirst.clear(); s->xfCount.clear();
     return CWP_OK;
+}
+extern "C" int cwp_server_set_scenes(cwp_server* s, const cwp_instance_desc* desc, int64_t n, const int32_t* first, int32_t nScenes) {
+    return with_room(s, [&] { return set_scenes(s, desc, n, first, nScenes); });
 }
 
 extern "C" int cwp_server_set_instance_xforms(cwp_server* s, const float* xforms, const int32_t* firstXf, const int32_t* nXf, int64_t n) {
@@ -697,7 +733,7 @@ extern "C" int cwp_server_set_instance_xforms(cwp_server* s, const float* xforms
     return CWP_OK;
 }
 
-extern "C" int cwp_server_set_envmaps(cwp_server* s, const cwp_envmap* maps, int32_t n) {
+static int set_envmaps(cwp_server* s, const cwp_envmap* maps, int32_t n) {
     CWPB_CHECK(s && n >= 0 && (n == 0 || maps), CWP_ERR_INVALID, "NULL argument");
     CWPB_CHECK(s->reqs.empty(), CWP_ERR_STATE, "environment maps change only while no request is queued or running");
     CWPB_CUDA(cudaSetDevice(s->device));
@@ -723,8 +759,11 @@ extern "C" int cwp_server_set_envmaps(cwp_server* s, const cwp_envmap* maps, int
     s->envs = built;
     return CWP_OK;
 }
+extern "C" int cwp_server_set_envmaps(cwp_server* s, const cwp_envmap* maps, int32_t n) {
+    return with_room(s, [&] { return set_envmaps(s, maps, n); });
+}
 
-extern "C" int cwp_server_set_textures(cwp_server* s, const cwp_texture* tex, int32_t nTex, const cwp_material_textures* mtex, int32_t nMtex,
+static int set_textures(cwp_server* s, const cwp_texture* tex, int32_t nTex, const cwp_material_textures* mtex, int32_t nMtex,
                                        const float* uvs, const float* tans) {
     CWPB_CHECK(s && nTex >= 0 && nMtex >= 0 && (nTex == 0 || tex) && (nMtex == 0 || mtex), CWP_ERR_INVALID, "NULL argument");
     CWPB_CHECK(s->reqs.empty(), CWP_ERR_STATE, "textures change only while no request is queued or running");
@@ -755,6 +794,10 @@ extern "C" int cwp_server_set_textures(cwp_server* s, const cwp_texture* tex, in
     cudaFree(s->dTexObj); cudaFree(s->dMtex); cudaFree(s->dUvs); cudaFree(s->dTans);
     s->texArrays = arrays; s->texObjs = objs; s->dTexObj = dObj; s->dMtex = dM; s->nMtex = used ? nMtex : 0; s->dUvs = dU; s->dTans = dT;
     return CWP_OK;
+}
+extern "C" int cwp_server_set_textures(cwp_server* s, const cwp_texture* tex, int32_t nTex, const cwp_material_textures* mtex, int32_t nMtex,
+                                       const float* uvs, const float* tans) {
+    return with_room(s, [&] { return set_textures(s, tex, nTex, mtex, nMtex, uvs, tans); });
 }
 
 __global__ void k_tex_sample(const cudaTextureObject_t* obj, const int* id, const float2* uv, float4* out, int64_t n) {
@@ -853,6 +896,22 @@ static int admission_budget(cwp_server* s, int64_t& avail) {
     return CWP_OK;
 }
 
+// stream-ordered pool memory for a request within the budget, or null where it does not fit (or the pool is too fragmented), not
+// even with the second shadow set given back
+static int take_memory(cwp_server* s, int64_t& avail, void** p, int64_t bytes) {
+    for (;;) {
+        const cudaError_t e = avail < bytes ? cudaErrorMemoryAllocation : cudaMallocFromPoolAsync(p, (size_t)bytes, s->pool, s->st);
+        if (e == cudaSuccess) { avail -= bytes; return CWP_OK; }
+        *p = nullptr;
+        if (e != cudaErrorMemoryAllocation) CWPB_CUDA(e);
+        if (avail >= bytes) cudaGetLastError();
+        bool freed = false;
+        if (int rc = give_back(s, freed)) return rc;
+        if (!freed) return CWP_OK;
+        if (int rc = admission_budget(s, avail)) return rc;
+    }
+}
+
 static int admit(cwp_server* s, bool& changed) {
     changed = false;
     if (s->pending.empty()) return CWP_OK;
@@ -865,11 +924,8 @@ static int admit(cwp_server* s, bool& changed) {
         if (!queried) { if (int rc = admission_budget(s, avail)) return rc; queried = true; }   // one query per step
         ServeRequest& q = s->reqs[s->pending.front()];
         const int64_t bytes = (int64_t)q.r.cam.w * q.r.cam.h * (int64_t)sizeof(float4);
-        if (avail < bytes) break;   // admission by free device memory
-        const cudaError_t e = cudaMallocFromPoolAsync((void**)&q.accum, (size_t)bytes, s->pool, s->st);   // stream-ordered, pooled
-        if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); q.accum = nullptr; break; }   // fragmentation: wait for frees
-        CWPB_CUDA(e);
-        avail -= bytes;
+        if (int rc = take_memory(s, avail, (void**)&q.accum, bytes)) return rc;
+        if (!q.accum) break;   // admission by free device memory: the request waits for others to finish
         CWPB_CUDA(cudaMemsetAsync(q.accum, 0, (size_t)bytes, s->st));
         SlotParams& P = s->hSlots[slot];
         P = SlotParams{};
@@ -885,14 +941,11 @@ static int admit(cwp_server* s, bool& changed) {
             const std::vector<float>& emT = q.emT; const std::vector<float>& emC = q.emC; const std::vector<float>& mlp = q.mlp;
             {
                 const size_t bT = emT.size() * sizeof(float), bC = (emC.size() * sizeof(float) + 15) & ~(size_t)15, bM = mlp.size() * sizeof(float);
-                const cudaError_t e2 = (int64_t)(bT + bC + bM) <= avail ? cudaMallocFromPoolAsync(&q.lights, bT + bC + bM, s->pool, s->st) : cudaErrorMemoryAllocation;
-                if (e2 == cudaErrorMemoryAllocation) {   // no room for the tables: the request waits with its image freed
-                    cudaGetLastError(); q.lights = nullptr;
+                if (int rc = take_memory(s, avail, &q.lights, (int64_t)(bT + bC + bM))) return rc;
+                if (!q.lights) {   // no room for the tables: the request waits with its image freed
                     CWPB_CUDA(cudaFreeAsync(q.accum, s->st)); q.accum = nullptr;
                     break;
                 }
-                CWPB_CUDA(e2);
-                avail -= (int64_t)(bT + bC + bM);
                 char* base = (char*)q.lights;   // pageable sources: staged before the calls return
                 CWPB_CUDA(cudaMemcpyAsync(base, emT.data(), bT, cudaMemcpyHostToDevice, s->st));
                 CWPB_CUDA(cudaMemcpyAsync(base + bT, emC.data(), emC.size() * sizeof(float), cudaMemcpyHostToDevice, s->st));
@@ -919,17 +972,6 @@ static int admit(cwp_server* s, bool& changed) {
         CWPB_CUDA(cudaMemcpyAsync(s->dSlots, s->hSlots, (size_t)s->O.max_requests * sizeof(SlotParams), cudaMemcpyHostToDevice, s->st));
         s->slotsDirty = false;
     }
-    return CWP_OK;
-}
-
-// adds a set's shadow times to the statistics once (waits for its end)
-static int take_shadow_times(cwp_server* s, int p) {
-    if (s->shadowTimed[p]) return CWP_OK;
-    s->shadowTimed[p] = true;
-    float d = 0, e = 0;
-    CWPB_CUDA(cudaEventSynchronize(s->evS[p][2]));
-    CWPB_CUDA(cudaEventElapsedTime(&d, s->evS[p][0], s->evS[p][2])); CWPB_CUDA(cudaEventElapsedTime(&e, s->evS[p][1], s->evS[p][2]));
-    s->info.shadow_ms += d; s->info.accum_ms += e;
     return CWP_OK;
 }
 

@@ -360,7 +360,9 @@ typedef struct cwp_server_options {
     int64_t max_paths;     /* paths in flight over all requests (default 8 Mi) */
     int32_t max_requests;  /* requests admitted at once (default 64; 1 for the plain form) */
     int32_t gd_energy;     /* glossy-diffuse energy compensation (default 1, as the reference's --gd_energy) */
-    int64_t hbm_reserve;   /* device bytes that admission leaves free (default 1 GiB) */
+    int64_t hbm_reserve;   /* device bytes that admission leaves free (default 1 GiB). Overlapped steps keep a second set of
+                              shadow rays (56 B per path of max_paths) in what lies above it at creation, and free it when a
+                              request or a table of cwp_server_set_* would not fit otherwise */
     int32_t device;
     int32_t regroup;       /* sort each step's continuations by request before tracing: 1 on, -1 off, 0 default (on) */
     int32_t policy;        /* new camera paths each step: 0 even share of the free path capacity among the requests with

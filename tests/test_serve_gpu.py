@@ -4,7 +4,7 @@ concurrent requests, continuous batching against the plain form, and admission b
 import numpy as np
 import pytest
 
-from conftest import golden
+from conftest import golden, only_free
 
 pytestmark = pytest.mark.gpu
 
@@ -447,3 +447,36 @@ def test_textured_request_matches_oracle(gpu, cwp, oracle, serving):
     assert abs(st_b.rays - cnt_b[0]) <= 5e-3 * cnt_b[0]
     with pytest.raises(cwp.CwpError):
         s.set_textures(imgs, cwp.material_textures([dict(base_color=9)]), uvs)   # texture id out of range
+
+
+def two_set_server(gpu, cwp, serving, paths, spare, **kw):
+    """a server whose second set of shadow rays (56 B a path) leaves `spare` bytes above its reserve"""
+    run_all(server(cwp, serving, max_paths=1 << 12, max_requests=1), requests(cwp, serving[5], 1, seed=4))   # kernels loaded
+    gpu.cuda.empty_cache()
+    before = gpu.cuda.mem_get_info()[0]
+    s = server(cwp, serving, max_paths=paths, hbm_reserve=1 << 50, **kw)   # more than any device has: one set
+    one = before - gpu.cuda.mem_get_info()[0]
+    del s
+    s = server(cwp, serving, max_paths=paths, hbm_reserve=gpu.cuda.mem_get_info()[0] - one - 56 * paths - spare, **kw)
+    assert before - gpu.cuda.mem_get_info()[0] >= one + 56 * paths - (8 << 20)   # it holds both
+    return s
+
+
+def test_second_shadow_set_gives_way_to_a_request(gpu, cwp, serving):
+    paths, boxes = 1 << 22, serving[5]
+    reqs = requests(cwp, boxes, 4, seed=21)
+    reqs.insert(2, requests(cwp, boxes, 1, seed=22, res=((2560, 1600),), spps=(1,))[0])   # an image of 65 MB
+    got = run_all(two_set_server(gpu, cwp, serving, paths, 32 << 20, max_requests=4), reqs)
+    alone = run_all(server(cwp, serving, max_paths=paths, max_requests=1), reqs)
+    for (a, sa), (b, sb) in zip(got, alone):
+        assert sa.rays == sb.rays and sa.shadow_rays == sb.shadow_rays and np.allclose(a, b, rtol=1e-4, atol=1e-5)
+
+
+def test_second_shadow_set_gives_way_to_a_table(gpu, cwp, serving):
+    s = two_set_server(gpu, cwp, serving, 1 << 22, 32 << 20, max_requests=4)
+    with only_free(gpu, 64 << 20):
+        s.set_envmaps([(np.full((1536, 3072, 3), 0.5, np.float32), 1.0)])   # 94 MB of tables
+    req = requests(cwp, serving[5], 1, seed=23)[0]
+    req.env = 0
+    (acc, st), = run_all(s, [req])
+    assert st.rays > 0 and np.all(np.isfinite(acc)) and acc[:, :3].sum() > 0
