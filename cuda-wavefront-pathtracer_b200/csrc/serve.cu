@@ -969,6 +969,7 @@ static int admit(cwp_server* s, bool& changed) {
         changed = true;
     }
     if (s->slotsDirty) {   // every admitted slot's parameters in one copy (the previous step's copies have completed)
+        CWPB_CUDA(cudaStreamSynchronize(s->st2));   // the previous step's shadow pass reads the slots it has entries of
         CWPB_CUDA(cudaMemcpyAsync(s->dSlots, s->hSlots, (size_t)s->O.max_requests * sizeof(SlotParams), cudaMemcpyHostToDevice, s->st));
         s->slotsDirty = false;
     }
@@ -1102,7 +1103,7 @@ extern "C" int cwp_server_step(cwp_server* s, int32_t* nActive, int32_t* nPendin
     s->info.admit_ms += now_ms(s) - admitStart;
     if (changed) {
         CWPB_CUDA(cudaStreamSynchronize(s->st));
-        CWPB_CUDA(cudaStreamSynchronize(s->st2));   // (the update's check and the traversals share the batch's status word)
+        // (and st2 is idle since the slots were copied: the update's check and the traversals share the batch's status word)
         const double t = now_ms(s);
         if (int rc = rebuild_tlas(s)) return rc;
         s->info.tlas_ms += now_ms(s) - t; s->info.tlas_rebuilds++;
