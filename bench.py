@@ -236,19 +236,26 @@ def port_scene(cwp, wl, variant, w=512, h=512, bounces=4):
 
 # DRAM bytes per launch of the frame kernels at the frame512 defaults, from a small-case capture scaled to the full
 # frame: the same frame at 16 spp (batch 16, 4.2 M paths per pass, path state 0.5 GB > L2), dram__bytes_read.sum +
-# dram__bytes_write.sum of every launch of one frame (one pass), per closest ray (k_trace_shade) or shadow ray
-# (k_shadow), times the full frame's rays over its 6 launches (summary and command in profiles/frame512_dram_traffic.txt).
-# Valid only for the configuration it was derived for.
-FRAME512_TRAFFIC = {"k_trace_shade": 1930e6, "k_shadow": 628e6}
+# dram__bytes_write.sum of every launch of one frame (one pass), per traced ray (camera rays, bounces and the rays beyond
+# the bounce limit together) or shadow ray, times the full frame's rays over its 6 or 5 launches (summary and command
+# in profiles/frame512_dram_traffic.txt). Valid only for the configuration it was derived for.
+FRAME512_TRAFFIC = {"trace": 1895e6, "shadow": 750e6}
 FRAME512_TRAFFIC_BINS = 128   # the build the capture ran on
 
 
-def frame_traffic(args, wl, variant, kernel):
+def trace_kernels(variant, traversal):
+    """the kernels that trace a frame's paths: camera rays, bounces, the rays beyond the bounce limit"""
+    first = "k_trace_shade_rf" if traversal == 1 else "k_trace_shade"
+    bounce = "k_bounce" if variant == 8 and traversal != 2 else first
+    return " + ".join(dict.fromkeys([first, bounce, "k_trace_shade" if traversal == 2 else "k_escape"]))
+
+
+def frame_traffic(args, wl, variant, group):
     captured = (args.workload == "frame512" and variant == 8 and args.spatial == 1e-3 and not args.spp and not args.batch and args.sort == 0
                 and args.graph == 1 and args.traversal == 0 and args.bins == FRAME512_TRAFFIC_BINS and args.stage_levels <= 0)
-    if not captured or kernel not in FRAME512_TRAFFIC:
+    if not captured:
         return {"traffic": None}
-    return {"traffic": FRAME512_TRAFFIC[kernel], "traffic_unit": "bytes per launch",
+    return {"traffic": FRAME512_TRAFFIC[group], "traffic_unit": "bytes per launch",
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the 16-spp frame (one pass, every launch), scaled by rays to the full frame (profiles/frame512_dram_traffic.txt)"}
 
 
@@ -256,14 +263,18 @@ NODE_BYTES = {2: 64, 4: 128, 8: 80}
 TRI_BYTES = 48   # Woop rows, an upper bound (the test reads row 2 first and rows 0/1 only past the t check)
 
 
-def onchip_bytes_frame(cwp, wl, mesh, bvh, variant, npix=1024):
+def onchip_bytes_frame(cwp, wl, mesh, bvh, variant, traversal, npix=1024):
     """Algorithmic on-chip bytes per ray of the frame (node visits x node size + triangle tests x 48 B), counted by
-    the oracle's traversal of the same tree over a band of pixels (part of the CPU-baseline leg)."""
+    the oracle's traversal of the same tree over a band of pixels (part of the CPU-baseline leg). The rays beyond the
+    bounce limit count with the any-hit traversal that k_escape runs."""
     sys.path.insert(0, os.path.join(ROOT, "tests"))
     from conftest import Oracle
     p = cwp.frame_params(mesh, wl["w"], wl["h"], bounces=wl["bounces"])
     N = wl["w"] * wl["h"]; pix0 = N // 2 - npix // 2
-    rc, st = Oracle().render_work(p, variant, 1, bvh, wl["bounces"], min(wl["spp"], 16), pix0, pix0 + npix)
+    orc = Oracle()
+    rc, st = orc.render_work(p, variant, 1, bvh, wl["bounces"], min(wl["spp"], 16), pix0, pix0 + npix)
+    if traversal != 2:
+        lim = orc.render_limit_work(); st[:2] += lim[2:] - lim[:2]
     nb = NODE_BYTES[variant]
     return dict(closest=(st[0] * nb + st[1] * TRI_BYTES) / max(rc[0], 1), shadow=(st[2] * nb + st[3] * TRI_BYTES) / max(rc[1], 1),
                 nodes_per_closest=st[0] / max(rc[0], 1), tris_per_closest=st[1] / max(rc[0], 1),
@@ -849,8 +860,9 @@ def main():
         # roofline of the dominant kernel (HBM: algorithmic path-state bytes per launch / its event-timed duration)
         tr_bytes = sum(STATE_BYTES * ((c_tot[d] if d > 0 else 0) + (c_tot[d + 1] if d + 1 < depths else 0) + s_tot[d]) for d in range(depths))
         sh_bytes = sum(STATE_BYTES * s_tot[d] for d in range(depths))
-        dom = "k_trace_shade" if tms.sum() >= sms.sum() else "k_shadow"
-        b, t = (tr_bytes, tms.sum()) if dom == "k_trace_shade" else (sh_bytes, sms.sum())
+        group = "trace" if tms.sum() >= sms.sum() else "shadow"
+        b, t = (tr_bytes, tms.sum()) if group == "trace" else (sh_bytes, sms.sum())
+        dom = trace_kernels(variant, args.traversal) if group == "trace" else "k_shadow_rf" if args.traversal == 1 else "k_shadow"
         achieved = b / (t * 1e-3) / 1e9 if t > 0 else 0.0
         out.update(metric=METRIC_FRAME, value=value, ms_per_step=max_ms / args.steps,
                    config={"workload": args.workload, "scene": f"{wl['scene']} ({mesh.n_tris} triangles, box field seed 1)", "references": len(bvh.order), "resolution": f"{w}x{h}",
@@ -867,7 +879,7 @@ def main():
                         "note": "scene uploaded once at init; each step renders and reads the w*h float4 accumulation buffer back into pinned host memory"},
                    gpu_launches=args.steps * (spp // K) * (1 + 2 * depths),   # pass begin and end, a trace per depth, a shadow pass for all but the last
                    roofline={"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                             "peak_kind": peak_kind, **frame_traffic(args, wl, variant, dom),
+                             "peak_kind": peak_kind, **frame_traffic(args, wl, variant, group),
                              "algorithmic": f"{STATE_BYTES} B of path state per queued ray read and per continuation/shadow ray written"})
         onchip = dict(kind="frame", closest=float(c_tot.sum()), shadow=float(s_tot.sum()), closest_ms=float(tms.sum()), shadow_ms=float(sms.sum()))
         ours_img = cwp.imageio.accum_to_image(r.read_accum(), w, h, spp)
@@ -984,10 +996,11 @@ def main():
         # on-chip roofline: oracle-counted node + triangle bytes per ray on the GPU's own tree, over the kernels' event
         # times, against the measured L2 read bandwidth (the scene is L2-resident, so this is the traversal's bound)
         if not wl.get("precision"):
-            ob = onchip_bytes_frame(cwp, wl, mesh, bvh, variant) if "rays" not in wl else onchip_bytes_trace(cwp, bvh, variant, o, d)
+            ob = onchip_bytes_frame(cwp, wl, mesh, bvh, variant, args.traversal) if "rays" not in wl else onchip_bytes_trace(cwp, bvh, variant, o, d)
             l2 = cwp.measure_l2_read(device=local)
             cb, sb = onchip["closest"] * ob["closest"], onchip["shadow"] * ob["shadow"]
-            kern = ("k_trace_shade", "k_shadow") if onchip["kind"] == "frame" else ("k_trace_closest", "k_trace_any")
+            kern = ((trace_kernels(variant, args.traversal), "k_shadow_rf" if args.traversal == 1 else "k_shadow") if onchip["kind"] == "frame"
+                    else ("k_trace_closest", "k_trace_any"))
             big = 0 if onchip["closest_ms"] >= onchip["shadow_ms"] else 1
             ach = [cb / (onchip["closest_ms"] * 1e-3) / 1e9, sb / (onchip["shadow_ms"] * 1e-3) / 1e9]
             out["roofline_onchip"] = {"bound": "l2", "kernel": kern[big], "achieved": ach[big], "peak": l2, "unit": "GB/s", "frac": ach[big] / l2,

@@ -543,7 +543,15 @@ static V3 a3(const float* a) { return v3(a[0], a[1], a[2]); }
 /* Traversal work of orc_render, for the on-chip roofline: [0] node visits and [1] triangle tests of closest-hit rays,
  * [2] and [3] of shadow rays. orc_render_stats(1, NULL) zeroes and enables the counters; (0, out) reads and disables. */
 static long long g_render_stats[4]; static int g_render_stats_on;
-void orc_render_stats(int on, long long* out) { if (out) memcpy(out, g_render_stats, sizeof g_render_stats); memset(g_render_stats, 0, sizeof g_render_stats); g_render_stats_on = on; }
+/* Of the rays beyond the bounce limit (depth > max_b), where only a miss counts: [0] and [1] their share of the closest-hit
+ * counters above, [2] and [3] what an any-hit traversal of them visits and tests. Zeroed with the others. */
+static long long g_render_limit[4];
+void orc_render_limit_stats(long long* out) { memcpy(out, g_render_limit, sizeof g_render_limit); }
+void orc_render_stats(int on, long long* out) {
+    if (out) memcpy(out, g_render_stats, sizeof g_render_stats);
+    if (on) memset(g_render_limit, 0, sizeof g_render_limit);
+    memset(g_render_stats, 0, sizeof g_render_stats); g_render_stats_on = on;
+}
 
 /* Renders samples [s_base, s_base + spp) of pixels [pix0, pix1) with `bounces` as the frame's depth limit
  * (depths 0 .. bounces + 1 are traced) and adds radiance sums to accum (float4 per pixel). Each path is traced
@@ -567,6 +575,12 @@ void orc_render(const OrcParams* P, int variant, int tri, const float* nodes, co
                 if (variant == 2) trav2((const V4*)nodes, (const V4*)tv, o, d, tmin, 0, tri, &t, &h, &u, &vv, g_render_stats_on ? &cs : NULL);
                 else trav8((const V4*)nodes, (const V4*)tv, o, d, tmin, 0, tri, &t, &h, &u, &vv, g_render_stats_on ? &cs : NULL);
                 g_render_stats[0] += cs.nodes; g_render_stats[1] += cs.tris;
+                if (g_render_stats_on && depth > P->max_b) {
+                    float at = 1e30f, au, av; int ah = -1; Stats as = {0, 0};
+                    if (variant == 2) trav2((const V4*)nodes, (const V4*)tv, o, d, tmin, 1, tri, &at, &ah, &au, &av, &as);
+                    else trav8((const V4*)nodes, (const V4*)tv, o, d, tmin, 1, tri, &at, &ah, &au, &av, &as);
+                    g_render_limit[0] += cs.nodes; g_render_limit[1] += cs.tris; g_render_limit[2] += as.nodes; g_render_limit[3] += as.tris;
+                }
                 if (h < 0) { V3 c = mulv(T, a3(P->sky)); accum[4 * pix] += c.x; accum[4 * pix + 1] += c.y; accum[4 * pix + 2] += c.z; break; }
                 if (depth > P->max_b) break;
                 V3 p = add(o, muls(d, t));

@@ -70,6 +70,8 @@ def _load_oracle():
     L.orc_bsdf_sample.argtypes = [C.c_void_p] * 4 + [C.c_int] + [C.c_void_p] * 6 + [C.c_long, C.c_void_p]
     L.orc_render_stats.restype = None
     L.orc_render_stats.argtypes = [C.c_int, C.c_void_p]
+    L.orc_render_limit_stats.restype = None
+    L.orc_render_limit_stats.argtypes = [C.c_void_p]
     L.orc_render_request.restype = C.c_long
     L.orc_render_request.argtypes = ([C.c_void_p, C.c_int, C.c_int] + [C.c_void_p] * 3 + [C.c_int] + [C.c_void_p] * 2 + [C.c_int, C.c_void_p, C.c_int, C.c_long, C.c_long, C.c_void_p, C.c_void_p]
                                      + [C.c_void_p] * 3 + [C.c_int, C.c_int] + [C.c_void_p] * 2 + [C.c_int] + [C.c_void_p] * 3 + [C.c_void_p] * 3 + [C.c_long, C.c_void_p, C.c_void_p])
@@ -251,6 +253,12 @@ class Oracle:
         _, rc = self.render(params, variant, tri, bvh, bounces, spp, 0, pix0, pix1)
         st = np.zeros(4, np.int64); self.L.orc_render_stats(0, st.ctypes.data)
         return rc, st
+
+    def render_limit_work(self):
+        """Of the last render_work, the rays beyond the bounce limit: [closest node visits, closest triangle tests (both
+        part of its counters), any-hit node visits, any-hit triangle tests]"""
+        st = np.zeros(4, np.int64); self.L.orc_render_limit_stats(st.ctypes.data)
+        return st
 
 
 @pytest.fixture(scope="session")

@@ -149,3 +149,15 @@ def test_frame_work_counters(cwp, oracle):
     assert np.array_equal(acc, acc2)
     rc1, st1 = oracle.render_work(p, 8, 1, b1, 2, 4, 0, 1024)
     assert st1[0] / rc1[0] < st0[0] / rc0[0]
+
+
+def test_frame_work_beyond_the_bounce_limit(cwp, oracle):
+    """The rays beyond the bounce limit are part of the closest-hit counters; as any-hit rays they visit fewer nodes"""
+    mesh = cwp.Mesh.box_field(300, 1)
+    b = cwp.Bvh(mesh, variant=8, bins=32, leaf=1)
+    p = cwp.frame_params(mesh, 32, 32, bounces=2)
+    _, st = oracle.render_work(p, 8, 1, b, 2, 4, 0, 1024)
+    lim = oracle.render_limit_work()
+    assert 0 < lim[2] < lim[0] < st[0] and 0 < lim[3] < lim[1] < st[1]
+    oracle.render_work(p, 8, 1, b, 0, 4, 0, 1024)   # depths 0 and 1 of 2 + 2 alone: none beyond the limit
+    assert np.all(oracle.render_limit_work() == 0)
