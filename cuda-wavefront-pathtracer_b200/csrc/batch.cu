@@ -43,7 +43,7 @@ template <int V, bool ANY>
 struct TwoLevel {
     // The state that both levels use (tmin, the hit's t, u, v) lives in blas alone, and the world ray's origin and direction are read
     // again from the queue on entering an instance, beside the instance's own record: 10 registers less across the traversal
-    // (spills of the 64-register kernels 244 -> 140 bytes closest, 212 -> 156 any).
+    // (spill stores of the 64-register CWBVH kernels 244 -> 108 bytes closest, 212 -> 124 any).
     float idx, idy, idz, ox, oy, oz; int hitTri, hitInst;
     int next, tsp, inst, budget;
     TravState<V, ANY, 0> blas;
@@ -146,8 +146,9 @@ __device__ __forceinline__ unsigned lane_mask_lt() { unsigned m; asm("mov.u32 %0
 // Persistent launch: each lane advances its ray one node visit at a time; a warp refetches rays (one atomic on the
 // queue cursor) once a.fetch of its lanes are idle. SMEM: the BLAS stack in shared memory, entry-major.
 template <int V, bool ANY, bool SMEM>
-// 64 registers (two 512-thread blocks per SM) with 132 bytes of spills: measured faster than 80 registers without
-// spills (1.83 vs 1.80 Grays/s on 64 scenes) or 128 registers (1.41); resident warps matter more than the spills
+// 64 registers (two 512-thread blocks per SM) with 108 (closest) and 124 (any) bytes of spills over a CWBVH: measured, when they
+// were 132, faster than 80 registers without spills (1.83 vs 1.80 Grays/s on 64 scenes) or 128 registers (1.41); resident warps
+// matter more than the spills
 __global__ void __launch_bounds__(kBatchMaxBlock, 2) k_batch_trace(const BatchArgs a) {
     typedef typename TravState<V, ANY, 0>::Stack LocalStack;
     typedef typename std::conditional<V == 8, uint2, int>::type Entry;
@@ -377,7 +378,8 @@ static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_
     // Triangle records, 3 float4 per triangle: (v0, local id), (v1, material), (v2, 0). The meshes go up as they are (half the
     // bytes of the records) and a kernel gathers them and checks vertex indices and coordinates. A mesh with more vertices than
     // corners (a part of a larger vertex array) leaves some unused for certain: its corners are taken out on the host and go up alone,
-    // so that parts sharing one array do not each bring the whole of it.
+    // so that parts sharing one array do not each bring the whole of it (64 parts of 5,000 triangles of one array of 1 M vertices:
+    // 6.6 ms to load, 44.9 with whole arrays; 64 meshes of 15,000 vertices each, which go up as they are, 3.7).
     {
         std::vector<RawMesh> raw(n);
         long long words = 0;

@@ -239,8 +239,8 @@ __device__ __forceinline__ float qbyte(unsigned w, int s) {
 // quarters of a visit's cycles (clock readings inside the kernel, 4.2 M incoherent rays over the 117k-triangle box field:
 // 1,580 cycles of node visit, 6,060 of leaf tests). test_leaves() lists the triangles of all lanes and hands them out 32 at a
 // time, one per lane, with the owner's ray read from shared memory: one fetch latency and one test for 16 triangles on
-// average. Measured there: 2,057 -> 1,670 us closest (12.1 -> 18.9 lanes per instruction, 449 -> 386 M instructions per
-// 1 M rays); rays and hits through shuffles instead of shared memory 1,781 us. Any-hit rays hit a quarter as many leaves
+// average. Measured there: 2,057 -> 1,709 us closest, with the paired slab tests of visit() 1,670 (12.1 -> 18.9 lanes per
+// instruction, 449 -> 386 M instructions per 1 M rays); rays and hits through shuffles instead of shared memory 1,781 us. Any-hit rays hit a quarter as many leaves
 // and stop at the first hit: for them the sharing measured no gain (434 vs 438 us) and their lanes test alone.
 struct LeafSet { unsigned hit = 0, m0 = 0, m1 = 0; int triBase = 0; };   // slots hit, the node's meta words, its first triangle
 template <bool UV>

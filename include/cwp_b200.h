@@ -462,6 +462,9 @@ int cwp_server_poll(cwp_server* s, int64_t* ids, int32_t cap, int32_t* n);
  * request's device memory is released. */
 int cwp_server_result(cwp_server* s, int64_t id, float* accum, cwp_request_stats* st);
 double cwp_server_clock_ms(const cwp_server* s);
+/* With overlapped steps a step's shadow pass runs beside the next step's closest hits: shadow_ms and accum_ms are spans that
+ * share the device with the other phases (the phases then add up to more than the device's busy time), and they are added when
+ * their set of shadow rays is used again or a request completes, up to two steps after the rays they belong to. */
 typedef struct cwp_server_info {
     int64_t steps, rays, shadow_rays, admissions, tlas_rebuilds;
     double closest_ms, shade_ms, shadow_ms, raygen_ms, tlas_ms, step_ms;   /* device time per phase (CUDA events), wall time of the steps */
