@@ -103,16 +103,19 @@ __global__ void k_seg_leaves(const float4* __restrict__ lo, const float4* __rest
     write_leaf(lo, hi, p, i, 2 * f - s + (i - f), nodes, count, C, bounds);
 }
 
-// Small segments (at most kSmallThreads * ITEMS primitives each: a scene's instances, a prop's triangles), one block per segment:
-// centroid bounds, keys, a stable block radix sort and the leaves in one launch. The general path takes 13 launches for the
-// same, 8 of them sort passes over all segments that each wait for the one before (rebuilding the TLAS of 7,864 instances in 8 scenes: 370 us with them, 300 without). Keys, order
-// and leaves are the same: the sort is stable on the same 54 bits, so equal keys keep the primitives' order.
-static constexpr int kSmallThreads = 1024;
-template <int ITEMS>
-__global__ void __launch_bounds__(kSmallThreads) k_seg_small(const float4* __restrict__ lo, const float4* __restrict__ hi, const int* __restrict__ segFirst,
+// Small segments (at most T * ITEMS primitives each: a scene's instances, a prop's triangles), one block per segment: centroid
+// bounds, keys, a stable block radix sort and the leaves in one launch. The general path takes 13 launches for the same, 8 of them
+// sort passes over all segments that each wait for the one before. Keys, order and leaves are the same: the sort is stable on the
+// same 54 bits, so equal keys keep the primitives' order. A block sorts T * ITEMS keys however many of them are its segment's, so
+// the block is the smallest that takes the largest segment. Device time of a TLAS rebuild, general path / this (us): 8 scenes of 30
+// instances 88 / 63, of 500 213 / 131, of 1024 259 / 179, of 4096 439 / 362; one of 1500 119 / 122 (1024 x 4 keys: 134), 1000
+// scenes of one 63 / 50 (blocks of 1024: 195) and of 30 394 / 277 (425).
+static constexpr int kSmallThreads = 1024, kTinyThreads = 128;
+template <int T, int ITEMS>
+__global__ void __launch_bounds__(T) k_seg_small(const float4* __restrict__ lo, const float4* __restrict__ hi, const int* __restrict__ segFirst,
                                                              unsigned long long* keysSorted, float4* nodes, int* count, int* C, int* bounds, int* counters) {
-    typedef cub::BlockRadixSort<unsigned long long, kSmallThreads, ITEMS, int> Sort;
-    __shared__ union { typename Sort::TempStorage sort; float box[6][kSmallThreads / 32]; } sh;
+    typedef cub::BlockRadixSort<unsigned long long, T, ITEMS, int> Sort;
+    __shared__ union { typename Sort::TempStorage sort; float box[6][T / 32]; } sh;   // T / 32 is a power of two (the second reduction reads it round and round)
     const int s = blockIdx.x, f = segFirst[s], m = segFirst[s + 1] - f, tid = threadIdx.x;
     if (tid == 0) counters[s] = 2 * f - s + m;   // internal nodes follow the segment's m leaves
     float c[ITEMS][3], mn[3] = { 3.4e38f, 3.4e38f, 3.4e38f }, mx[3] = { -3.4e38f, -3.4e38f, -3.4e38f };
@@ -135,7 +138,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_seg_small(const float4* __res
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        mn[k] = sh.box[k][tid & 31]; mx[k] = sh.box[3 + k][tid & 31];
+        mn[k] = sh.box[k][tid & (T / 32 - 1)]; mx[k] = sh.box[3 + k][tid & (T / 32 - 1)];
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) { mn[k] = fminf(mn[k], __shfl_xor_sync(kFull, mn[k], off)); mx[k] = fmaxf(mx[k], __shfl_xor_sync(kFull, mx[k], off)); }
     }
@@ -333,8 +336,12 @@ int SegBuilder::build(const float4* lo, const float4* hi, int64_t n64, const int
     const int g = (n + 255) / 256;
     int most = 0;
     for (int s = 0; s < nSeg; s++) most = segFirstHost[s + 1] - segFirstHost[s] > most ? segFirstHost[s + 1] - segFirstHost[s] : most;
-    if (most <= kSmallThreads) k_seg_small<1><<<nSeg, kSmallThreads, 0, st>>>(lo, hi, segFirst, keysSorted, nodes, count, clusters, bounds, counters);
-    else if (most <= 4 * kSmallThreads) k_seg_small<4><<<nSeg, kSmallThreads, 0, st>>>(lo, hi, segFirst, keysSorted, nodes, count, clusters, bounds, counters);
+#define CWPB_SMALL(T, ITEMS) k_seg_small<T, ITEMS><<<nSeg, T, 0, st>>>(lo, hi, segFirst, keysSorted, nodes, count, clusters, bounds, counters)
+    if (most <= kTinyThreads) CWPB_SMALL(kTinyThreads, 1);
+    else if (most <= kSmallThreads) CWPB_SMALL(kSmallThreads, 1);
+    else if (most <= 2 * kSmallThreads) CWPB_SMALL(kSmallThreads, 2);
+    else if (most <= 4 * kSmallThreads) CWPB_SMALL(kSmallThreads, 4);
+#undef CWPB_SMALL
     else {
         k_seg_init<<<(nSeg + 127) / 128, 128, 0, st>>>(cbox, counters, segFirst, nSeg);
         k_seg_bounds<<<g, 256, 0, st>>>(lo, hi, n, segFirst, nSeg, cbox);

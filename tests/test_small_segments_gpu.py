@@ -30,3 +30,9 @@ def test_small_segments_build_the_general_tree(gpu, cwp, sizes, kind):
         for i in range(len(meshes)):   # the leaf order of each mesh's triangles, which the whole tree decides
             mine = [t[t[:, 1, 3].view(np.int32) == i] for t in (a, b)]
             assert np.array_equal(mine[0].view(np.uint32), mine[1].view(np.uint32)), (width, i)
+
+
+@pytest.mark.parametrize("sizes", [(127, 128, 1), (129, 2), (2047, 2048), (2049, 1)])   # around the other block sizes
+@pytest.mark.parametrize("kind", ["random", "pairs"])
+def test_block_sizes_build_the_general_tree(gpu, cwp, sizes, kind):
+    test_small_segments_build_the_general_tree(gpu, cwp, sizes, kind)
