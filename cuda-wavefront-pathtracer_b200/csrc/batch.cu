@@ -344,6 +344,7 @@ static int host_build(cwp_batch* b, const cwp_mesh_view* meshes, int n, float sp
     return CWP_OK;
 }
 
+static constexpr long long kStageWords = 16384;   // a mesh of up to 64 KB goes up with its neighbours (batch_create)
 static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_options* opt, cwp_batch* b) {
     b->device = opt ? opt->device : 0;
     b->leaf = opt && opt->leaf > 0 ? opt->leaf : 4;
@@ -401,17 +402,33 @@ static int batch_create(const cwp_mesh_view* meshes, int32_t n, const cwp_batch_
         else { CWPB_CUDA(cudaMalloc(&own, bytes)); placeRaw(Carver(own)); }
         cudaError_t e = cudaMemcpyAsync(dRaw, raw.data(), (size_t)n * sizeof(RawMesh), cudaMemcpyHostToDevice, b->st);
         if (e == cudaSuccess) e = cudaMemsetAsync(dBad, 0xff, sizeof(unsigned long long), b->st);
+        // Small meshes are put together on the host and go up in one copy: a copy call costs 3 us, the words of a small mesh less
+        // (loading 900 meshes of 12 triangles 12.9 -> 8.3 ms, of 100 14.4 -> 10.3, 64 of 500 4.3 -> 3.4, 200 of 1365 6.4 -> 6.2).
+        // The sources are pageable, so each is staged before its copy call returns
+        std::vector<unsigned> stage; long long stageAt = 0;
+        auto flush = [&]() {
+            if (e == cudaSuccess && !stage.empty()) e = cudaMemcpyAsync(dWords + stageAt, stage.data(), stage.size() * 4, cudaMemcpyHostToDevice, b->st);
+            stage.clear();
+        };
         for (int m = 0; m < n && e == cudaSuccess; m++) {
             const cwp_mesh_view& v = meshes[m];
-            std::vector<float> corners;   // (a pageable source: staged before the copy call returns)
+            std::vector<float> corners;
             if (raw[m].face < 0) {
                 corners.assign((size_t)9 * v.n_tris, NAN);   // NaN where the index is out of range: the kernel finds the corner, the check below says why
                 for (int64_t c = 0; c < 3 * v.n_tris; c++) { const int vi = v.faces[c]; if (vi >= 0 && vi < v.n_verts) memcpy(&corners[3 * c], v.verts + 3 * (size_t)vi, 12); }
             }
-            e = cudaMemcpyAsync(dWords + raw[m].vert, raw[m].face < 0 ? corners.data() : v.verts, (size_t)raw[m].nVerts * 12, cudaMemcpyHostToDevice, b->st);
-            if (e == cudaSuccess && raw[m].face >= 0) e = cudaMemcpyAsync(dWords + raw[m].face, v.faces, (size_t)v.n_tris * 12, cudaMemcpyHostToDevice, b->st);
-            if (e == cudaSuccess && v.face_mat) e = cudaMemcpyAsync(dWords + raw[m].mat, v.face_mat, (size_t)v.n_tris * 4, cudaMemcpyHostToDevice, b->st);
+            const bool small = (m + 1 < n ? raw[m + 1].vert : words) - raw[m].vert <= kStageWords;
+            if (!small || stage.size() > 16 * (size_t)kStageWords) flush();
+            if (stage.empty()) stageAt = raw[m].vert;
+            auto up = [&](long long at, const void* src, long long count) {   // the mesh's arrays follow one another in dWords, as in the stage
+                if (small) stage.insert(stage.end(), static_cast<const unsigned*>(src), static_cast<const unsigned*>(src) + count);
+                else if (e == cudaSuccess) e = cudaMemcpyAsync(dWords + at, src, (size_t)count * 4, cudaMemcpyHostToDevice, b->st);
+            };
+            up(raw[m].vert, raw[m].face < 0 ? corners.data() : v.verts, 3 * raw[m].nVerts);
+            if (raw[m].face >= 0) up(raw[m].face, v.faces, 3 * v.n_tris);
+            if (v.face_mat) up(raw[m].mat, v.face_mat, v.n_tris);
         }
+        flush();
         unsigned long long bad = ~0ull;
         if (e == cudaSuccess) { gather_triangles(dWords, dRaw, n, b->nTris, b->triV, dBad, b->st); e = cudaGetLastError(); }
         if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, dBad, sizeof bad, cudaMemcpyDeviceToHost, b->st);

@@ -47,14 +47,14 @@ def test_first_bad_corner_is_named(gpu, cwp, mesh, tri, corner, what, builder):
     assert text in str(e.value)
 
 
-def parts(n_verts, counts):
+def parts(n_verts, counts, half=5.0, size=None):
     """meshes that each use a few vertices of one array of n_verts, from its start to its end, and the same meshes compacted"""
     big = np.zeros((n_verts, 3), np.float32)   # (pages that nothing touches take no memory)
     rng = np.random.default_rng(5)
     shared, alone = [], []
     for i, n in enumerate(counts):
         at = (n_verts - 3 * n) * i // max(1, len(counts) - 1)
-        big[at:at + 3 * n] = rng.uniform(-5, 5, (3 * n, 3))
+        big[at:at + 3 * n] = rng.uniform(-half, half, (3 * n, 3)) if size is None else (rng.uniform(-half, half, (n, 1, 3)) + rng.uniform(-size, size, (n, 3, 3))).reshape(-1, 3)
         f = np.arange(3 * n, dtype=np.int32).reshape(n, 3)
         mat = np.full(n, i, np.int32)
         shared.append((big, f + at, mat, None)); alone.append((big[at:at + 3 * n], f, mat, None))
@@ -93,3 +93,25 @@ def test_first_bad_corner_of_a_part(gpu, cwp, what):
         cwp.Batch(shared)
     assert e.value.code == cwp.ERR_INVALID
     assert (f"mesh 1: non-finite vertex {f[7, 1]}" if what == "nan" else f"mesh 1 triangle 7: vertex index {f[7, 1]} out of range") in str(e.value)
+
+
+@pytest.mark.parametrize("sizes", [(5000, 3, 6000, 1, 2), (1200,) * 30 + (4000,)])   # meshes that go up alone and, before, after and between them, together
+@pytest.mark.parametrize("builder", [0, 1])
+def test_small_meshes_between_large_ones(gpu, cwp, sizes, builder):
+    rng = np.random.default_rng(7)
+    meshes = []
+    for i, n in enumerate(sizes):
+        v = (rng.uniform(-50, 50, (n, 1, 3)) + rng.uniform(-0.2, 0.2, (n, 3, 3))).astype(np.float32)
+        meshes.append((v.reshape(-1, 3), np.arange(3 * n, dtype=np.int32).reshape(n, 3), rng.integers(0, 9, n).astype(np.int32), None))
+    b = cwp.Batch(meshes, builder=builder)
+    for width in (2, 4, 8):
+        rec = b.download(width)[1].reshape(-1, 3, 4)
+        got = np.concatenate([rec[:, 0, :3], rec[:, 1, :3], rec[:, 2, :3], rec[:, :2, 3].copy().view(np.int32).astype(np.float32)], 1)
+        want = np.concatenate([np.concatenate([(t := v.reshape(-1, 3, 3))[:, 0], t[:, 1] - t[:, 0], t[:, 2] - t[:, 0], np.arange(len(f))[:, None], m[:, None]], 1)
+                               for v, f, m, _ in meshes]).astype(np.float32)
+        assert np.array_equal(want[np.lexsort(want.T)], got[np.lexsort(got.T)])
+
+
+def test_large_and_small_parts(gpu, cwp):
+    shared, alone = parts(200000, (2500, 3, 3000, 2), 50, 0.2)   # 90 KB of corners and more alone, the small ones together
+    assert same_layouts(cwp.Batch(shared), cwp.Batch(alone))
