@@ -327,11 +327,12 @@ static int launch_batch(const DeviceScene& s, const float4* o, const float4* d, 
         for (long long at = 0; at < n; at += 1ll << 30) {
             const int m = (int)std::min<long long>(n - at, 1ll << 30);
             float4* const hits = ANY ? nullptr : (float4*)out + at; int* const occ = ANY ? (int*)out + at : nullptr;
+            const int grid = std::min(refillGrid, m);   // no more blocks than rays: one ray 10.3 -> 7.2 us, 2 to 100 rays 1 to 2 us less
             CWPB_CUDA(cudaMemsetAsync(fetch, 0, sizeof(unsigned long long), st));
-#define CWPB_R(VV, TT) k_trace_rf<VV, TT, ANY><<<refillGrid, kBatchBlock, 0, st>>>(s.nodes, tv0, o + at, d + at, hits, occ, m, fetch, err)
+#define CWPB_R(VV, TT) k_trace_rf<VV, TT, ANY><<<grid, kBatchBlock, 0, st>>>(s.nodes, tv0, o + at, d + at, hits, occ, m, fetch, err)
             if (s.precise) {   // closest hits share their triangle tests over the warp; any-hit rays keep their own
                 if (ANY) CWPB_R(16, 1);
-                else k_trace_prec_rf<<<refillGrid, kBatchBlock, 0, st>>>(s.nodes, tv0, o + at, d + at, hits, m, fetch, err);
+                else k_trace_prec_rf<<<grid, kBatchBlock, 0, st>>>(s.nodes, tv0, o + at, d + at, hits, m, fetch, err);
             }
             else if (s.variant == 2) { if (s.tri) CWPB_R(2, 1); else CWPB_R(2, 0); }
             else { if (s.tri) CWPB_R(8, 1); else CWPB_R(8, 0); }
