@@ -169,6 +169,10 @@ __global__ void __launch_bounds__(kBatchBlock) k_trace_any(const float4* __restr
 static constexpr int kRefillBatch = CWPB_BATCH_REFILL;
 static constexpr int kRefillShare = 6;   // with shared triangle tests (2 / 4 / 6 / 8 / 12 / 16 idle lanes: 1769 / 1690 / 1670 / 1683 / 1764 / 1896 us
                                          // for 4.2 M incoherent closest hits)
+// The precision form's any-hit rays have no form for a warp's last rays, so even shares pay only while few rays of a warp wait for one
+// another: against whole fetches, at 2 / 3 / 5 / 7 / 9 / 13 rays a warp (5 k to 60 k rays, mean over trees of 3.6 k to 117 k triangles and
+// two ray lengths) 1.21 / 1.15 / 1.06 / 0.98 / 0.96 / 0.96 times as fast. FP32 kernels gain or keep at every share.
+static constexpr int kSharePrec = 5;
 __device__ __forceinline__ unsigned lane_lt() { unsigned m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
 
 template <int V, int TRI, bool ANY>
@@ -181,7 +185,8 @@ __global__ void __launch_bounds__(kBatchBlock, 8) k_trace_rf(const float4* __res
     int e = 0;
     TravState<V, ANY, TRI> ray; typename TravState<V, ANY, TRI>::Stack stack;
     int k = -1; bool fin = false, drained = false;
-    const int cap = warp_share(n, gridDim.x * (kBatchBlock / 32));
+    int cap = warp_share(n, gridDim.x * (kBatchBlock / 32));
+    if (V == 16 && cap > kSharePrec) cap = 32;
     for (;;) {
         if (fin) {
             if (ANY) __stcs(occ + k, ray.hitTri);
