@@ -572,7 +572,7 @@ struct cwp_renderer {
     // shadow rays of a depth run on a second stream while the next depth is traced (see enqueue_passes)
     bool beside = false; cudaStream_t st2 = nullptr; cudaEvent_t traced = nullptr, shadowed = nullptr;
     cudaGraphExec_t gexec = nullptr; int gSpp = -1;
-    int gridTrace = 0, gridTrace0 = 0, gridShadow = 0, nSM = 0; bool refill = false, refillShadow = false;
+    int gridTrace = 0, gridTrace0 = 0, gridShadow = 0, nSM = 0; bool refill = false, refillShadow = false, fewTris = false;
     int staged = 0;   // CWBVH nodes staged in each traversal block's shared memory (0 = none)
     std::vector<void*> allocs;
     double vramMB = 0; std::string gpuName;
@@ -624,6 +624,7 @@ template <int V, int TRI, bool STAGE = false> int launch_depth(cwp_renderer* r, 
         if (rf && !escape) {
             if (a.depth == 0 && r->O.traversal == 1) k_trace_shade_rf<V, TRI, true, STAGE><<<gt0, 128, sm, r->st>>>(a, r->P);
             else if (a.depth == 0) k_trace_shade<V, TRI, true, STAGE><<<gt0, 128, sm, r->st>>>(a, r->P);
+            else if (r->fewTris) k_trace_shade<V, TRI, false, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
             else if constexpr (V == 8) k_bounce<TRI, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
             else k_trace_shade_rf<V, TRI, false, STAGE><<<gt, 128, sm, r->st>>>(a, r->P);
         }
@@ -682,6 +683,11 @@ int ensure_events(cwp_renderer* r, int passes) {
     r->evPasses = passes;
     return CWP_OK;
 }
+
+// Bounces over a CWBVH of up to this many leaf triangles run one fetch per warp: rays that visit few nodes finish together, and
+// k_bounce's sharing and listing cost more than they save. The four bounces of 1280x720x4, k_bounce / one fetch (us): 362 triangles
+// 327 / 258, 3,602 1,149 / 1,042, 6,002 1,658 / 1,576, 8,402 2,022 / 1,992, 12,290 2,467 / 2,537, 117,002 4,235 / 4,980.
+static constexpr int64_t kFewTris = 8192;
 
 // All passes of a frame with device-side queue lengths and persistent grids (the captured sequence). Every launch of a small
 // pass ends in a tail: its queue is empty and a few long rays hold the GPU. With r->beside the shadow pass of a depth is a
@@ -838,6 +844,7 @@ extern "C" int cwp_renderer_init(cwp_renderer* r, const cwp_params* p, const cwp
     // latency) run faster per 32-ray batch
     r->refill = o->traversal == 1 || (o->traversal == 0 && V == 8);
     r->refillShadow = o->traversal == 1;
+    r->fewTris = o->traversal == 0 && V == 8 && s->n_tris <= kFewTris;
     // CWBVH top levels staged in shared memory: stage_levels 0 = the default, < 0 none, 1..3 levels 0..L (at most
     // kMaxStagedNodes nodes)
     CWPB_CHECK(o->stage_levels <= 3, CWP_ERR_INVALID, "stage_levels %d is above 3", o->stage_levels);

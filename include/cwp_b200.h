@@ -173,8 +173,8 @@ typedef struct cwp_render_options {
     int32_t block;        /* threads per block of the traversal kernels (0 = 128) */
     int32_t device;       /* CUDA device ordinal */
     int32_t profile;      /* 1: CUDA event pair around every kernel launch (also inside the graph), see cwp_renderer_depth_stats */
-    int32_t traversal;    /* 0 auto (refill for CWBVH bounces and, in every layout, for the any-hit traversal of the rays beyond the
-                             bounce limit), 1 persistent lanes with dynamic refill everywhere, 2 everywhere one fetch of up to 32
+    int32_t traversal;    /* 0 auto (refill for CWBVH bounces over more than 8,192 leaf triangles and, in every layout, for the
+                             any-hit traversal of the rays beyond the bounce limit), 1 persistent lanes with dynamic refill everywhere, 2 everywhere one fetch of up to 32
                              rays per warp at a time, traversed to the end */
     int32_t sort;         /* continuation rays regrouped before each bounce: 0 off, 1 by direction octant, 2 by octant and a 4x4x4 origin cell */
     int32_t stage_levels; /* CWBVH: levels 0..L of the tree copied into every traversal block's shared memory (L = 1..3, at most

@@ -59,3 +59,17 @@ def test_fewer_bounces_than_the_limit(gpu, cwp, oracle, variant, traversal):
     want, counts = oracle.render(p, variant, 1, bvh, 4, 8)
     assert cwp.imageio.psnr(acc[:, :3] / 8, want[:, :3] / 8) >= 60.0
     assert abs(st.rays - counts[0]) <= 1e-3 * counts[0] and abs(st.shadow_rays - counts[1]) <= 1e-3 * counts[1]
+
+
+@pytest.mark.parametrize("boxes", [682, 683])   # 8,186 and 8,198 triangles: either side of the line between the bounce kernels
+@pytest.mark.parametrize("spatial", [0.0, 1e-3])
+def test_bounce_kernels_on_either_side_of_the_line(gpu, cwp, oracle, boxes, spatial):
+    mesh, bvh = cwp.scene(boxes, variant=8, bins=32, spatial=spatial)
+    p = cwp.frame_params(mesh, 40, 20, bounces=3)
+    st, acc = render(cwp, p, bvh, 8, 8, batch=8, bounces=3)
+    s1, refill = render(cwp, p, bvh, 8, 8, batch=8, bounces=3, traversal=1)
+    assert (st.rays, st.shadow_rays) == (s1.rays, s1.shadow_rays)
+    assert same_sums(acc, refill, 8 * 5 * 2)
+    want, counts = oracle.render(p, 8, 1, bvh, 3, 8)
+    assert cwp.imageio.psnr(acc[:, :3] / 8, want[:, :3] / 8) >= 60.0
+    assert abs(st.rays - counts[0]) <= 1e-3 * counts[0] and abs(st.shadow_rays - counts[1]) <= 1e-3 * counts[1]
