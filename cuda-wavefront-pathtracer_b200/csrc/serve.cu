@@ -558,7 +558,7 @@ static int take_shadow_times(cwp_server* s, int p) {
 // when something else needs the memory; true when there was a set to free.
 static int give_back(cwp_server* s, bool& freed) {
     freed = false;
-    if (!s->beside) return CWP_OK;
+    if (!s->second) return CWP_OK;
     CWPB_CUDA(cudaStreamSynchronize(s->st)); CWPB_CUDA(cudaStreamSynchronize(s->st2));
     for (int p = 0; p < 2; p++) if (int rc = take_shadow_times(s, p)) return rc;
     s->beside = false; s->par = 0;
@@ -667,7 +667,9 @@ static int server_create(cwp_batch* b, const cwp_material* mats, int n, const in
         uint64_t keep = UINT64_MAX;   // never hand freed images back to the driver between steps
         CWPB_CUDA(cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     }
-    // the second shadow set, where it leaves the reserve untouched and steps overlap (otherwise each waits for its own shadow pass)
+    // the second shadow set, where it leaves the reserve untouched and steps overlap; a step that waits for its own shadow pass needs one
+    // set for it to run beside the regrouping
+    s->beside = !s->overlap;
     if (s->overlap) {
         size_t freeB = 0, totalB = 0;
         CWPB_CUDA(cudaMemGetInfo(&freeB, &totalB));
@@ -1046,7 +1048,7 @@ static int launch_step(cwp_server* s) {
     CWPB_CUDA(cudaEventRecord(s->ev[1], s->st));
     CWPB_CUDA(cudaEventRecord(s->ev[2], s->st));
     CWPB_CUDA(cudaEventRecord(s->ev[3], s->st));
-    if (s->beside) s->par ^= 1;
+    if (s->second) s->par ^= 1;
     const int p = s->par;
     const cudaStream_t ss = s->beside ? s->st2 : s->st;   // the shadow pass's stream
     int* const cnt = s->cnt[p];
