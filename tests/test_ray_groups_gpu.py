@@ -35,3 +35,24 @@ def test_small_batches_bitexact_vs_oracle(gpu, cwp, oracle, rays, tri, spatial):
         gpu.cuda.synchronize(); acc.status()
         assert np.array_equal(hits.cpu().numpy().view(np.uint32), want[:n]), n
         assert np.array_equal(occ.cpu().numpy(), want_any[:n]), n
+
+
+def test_precision_shares_bitexact_vs_oracle(gpu, cwp, oracle, rays):
+    """precision any-hit rays: even shares up to five rays a warp, whole fetches above; closest hits beside them"""
+    _, bvh = cwp.scene(1024, variant=8, bins=32)
+    acc = cwp.Accel(bvh)
+    acc.set_precision(1)
+    o, d = rays
+    warps = gpu.cuda.get_device_properties(0).multi_processor_count * 8 * 4
+    sizes = [1, 3, warps - 1, 5 * warps, 5 * warps + 1, 32 * warps]
+    assert sizes[-1] <= len(o)
+    want = oracle.trace_prec(bvh.nodes, bvh.verts, o, d).view(np.uint32)
+    want_any = oracle.trace_prec(bvh.nodes, bvh.verts, o, d, any_hit=True)
+    to, td = gpu.from_numpy(o).cuda(), gpu.from_numpy(d).cuda()
+    for n in sizes:
+        hits = gpu.full((n, 4), -7.0, dtype=gpu.float32, device="cuda"); occ = gpu.full((n,), -7, dtype=gpu.int32, device="cuda")
+        acc.trace_closest(to.data_ptr(), td.data_ptr(), hits.data_ptr(), n)
+        acc.trace_any(to.data_ptr(), td.data_ptr(), occ.data_ptr(), n)
+        gpu.cuda.synchronize(); acc.status()
+        assert np.array_equal(hits.cpu().numpy().view(np.uint32), want[:n]), n
+        assert np.array_equal(occ.cpu().numpy(), want_any[:n]), n
